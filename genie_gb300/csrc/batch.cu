@@ -22,6 +22,8 @@ struct genie_batch {
     cudaStream_t stream = nullptr;
     cudaGraphExec_t gexec = nullptr;
     bool graph_valid = false;
+    bool graph_planes = false;       // the graph was captured with the index's planes
+    uint32_t need = 0, graph_need = 0;   // LaunchNeed of the batches staged so far, and of the graph
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     cudaEvent_t stage_ev[kStages + 1] = {};
     // pinned staging
@@ -76,21 +78,28 @@ DevQueries device_queries(const genie_batch *b) {
 int enqueue(genie_batch *b, cudaStream_t s) {
     DeviceContext &ctx = device_context(b->ix->device);
     const DevQueries q = device_queries(b);
+    const DevIndex d = index_view(b->ix, b->tuning);     // directories built before a capture
+    if (d.planes && !b->ws.planes.p) {                   // earlier launches may still use the scratch
+        cudaError_t e = cudaDeviceSynchronize();
+        if (!e) e = b->ws.reserve_planes(b->cfg.max_queries);
+        if (e) return cuda_fail(e, "batch buffers");
+        b->graph_valid = false;
+    }
     const Work w = b->ws.view(b->cfg.max_queries, true);
     if (!b->cfg.use_graph) {
         // direct launches, with an event after every stage for per-kernel timing
-        b->last_kernels = launch_match(index_view(b->ix, b->tuning), q, w, b->tuning, ctx.num_sms, s, b->stage_ev);
+        b->last_kernels = launch_match(d, q, w, b->tuning, ctx.num_sms, s, b->stage_ev, b->need);
         cudaError_t e = cudaGetLastError();
         return e ? cuda_fail(e, "batch launch") : GENIE_OK;
     }
-    if (!b->graph_valid) {
+    if (!b->graph_valid || b->graph_planes != (d.planes != nullptr) || (d.planes && b->graph_need != b->need)) {
+        b->graph_valid = false;
         if (b->gexec) cudaGraphExecDestroy(b->gexec);
         b->gexec = nullptr;
         cudaGraph_t g = nullptr;
-        const DevIndex d = index_view(b->ix, b->tuning);     // directories built before the capture
         cudaError_t e = cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal);
         if (e) return cuda_fail(e, "graph capture");
-        b->last_kernels = launch_match(d, q, w, b->tuning, ctx.num_sms, b->stream);
+        b->last_kernels = launch_match(d, q, w, b->tuning, ctx.num_sms, b->stream, nullptr, b->need);
         cudaError_t le = cudaGetLastError();
         e = cudaStreamEndCapture(b->stream, &g);
         if (le) {
@@ -102,6 +111,8 @@ int enqueue(genie_batch *b, cudaStream_t s) {
         cudaGraphDestroy(g);
         if (e) return cuda_fail(e, "graph instantiate");
         b->graph_valid = true;
+        b->graph_planes = d.planes != nullptr;
+        b->graph_need = b->need;
     }
     cudaError_t e = cudaGraphLaunch(b->gexec, s);
     return e ? cuda_fail(e, "graph launch") : GENIE_OK;
@@ -120,6 +131,8 @@ int stage_async(genie_batch *b, const genie_queries *q, cudaStream_t s) {
         const uint32_t k = q->k ? q->k[i] : q->uniform_k;
         if (k > b->cfg.max_k) return fail(GENIE_ERR_INVALID_ARG, "k=%u exceeds the batch capacity %u", k, b->cfg.max_k);
     }
+    note_search(b->ix, q);
+    b->need |= launch_need(b->ix, q);
     // The caller's item arrays are uploaded from where they are: a copy from
     // pageable memory returns once the source may be reused, and on a
     // coherently attached host it moves the bytes without a staging memcpy,

@@ -104,11 +104,18 @@ cudaError_t Workspace::reserve(int64_t Q, int64_t items, int64_t units, int64_t 
     return cudaSuccess;
 }
 
+cudaError_t Workspace::reserve_planes(int64_t Q) {
+    // a few queries of many tiles write more than 64 parts' keys each
+    cudaError_t e = scratch.reserve(8 << 20);
+    if (!e) e = planes.reserve((size_t)Q * (8 + 256 * 4 + 4) + 64);
+    return e;
+}
+
 void Workspace::release() {
     DevBuf *all[] = {&item_off, &dim, &low, &up, &weight, &weighted, &k, &out_off, &item_k0, &item_nk,
                      &item_inc, &span_start,
                      &span_len, &inc, &qinfo, &work, &ctr, &qstate, &done, &lb, &part_cnt, &scratch,
-                     &out_ids, &out_counts, &out_scores, &counters, &unit_key};
+                     &out_ids, &out_counts, &out_scores, &counters, &unit_key, &planes};
     for (DevBuf *b : all) b->release();
 }
 
@@ -130,6 +137,10 @@ Work Workspace::view(int64_t Q, bool scores) const {
     w.lb = (uint32_t *)lb.p;
     w.part_cnt = (uint32_t *)part_cnt.p;
     w.scratch = (uint64_t *)scratch.p;
+    w.scratch_keys = (int64_t)(scratch.bytes / 8);
+    w.pl_hist = (uint32_t *)planes.p;
+    w.lbk = planes.p ? (uint64_t *)(w.pl_hist + Q * 256) : nullptr;
+    w.pl_cur = planes.p ? (uint32_t *)(w.lbk + Q) : nullptr;
     w.max_parts = kMaxDenseParts;
     w.out_ids = (uint32_t *)out_ids.p;
     w.out_counts = (uint32_t *)out_counts.p;
@@ -285,6 +296,7 @@ int run_search(genie_index *ix, const genie_queries *q, const std::vector<int64_
     if (ix->sub_shift >= 0) return subseq_search(ix, q, out_off, n_items, out_ids, out_counts, out_scores, sync);
     const int64_t Q = q->n_queries;
     const int64_t sumk = out_off[Q];
+    note_search(ix, q);
     Workspace &ws = ix->ws;
     cudaError_t e = ws.reserve(Q, n_items, count_units(ix->host, q), sumk);
     if (e) return cuda_fail(e, "search workspace");
@@ -314,9 +326,11 @@ int run_search(genie_index *ix, const genie_queries *q, const std::vector<int64_
     dq.uniform_k = q->uniform_k;
     dq.out_off = (const int64_t *)ws.out_off.p;
     dq.dyn = nullptr;
-    Work w = ws.view(Q, out_scores != nullptr);
     DeviceContext &ctx = device_context(ix->device);
-    ix->last_launches = launch_match(index_view(ix, ix->tuning), dq, w, ix->tuning, ctx.num_sms, s);
+    const DevIndex d = index_view(ix, ix->tuning);
+    if (d.planes && (e = ws.reserve_planes(Q))) return cuda_fail(e, "search workspace");
+    Work w = ws.view(Q, out_scores != nullptr);
+    ix->last_launches = launch_match(d, dq, w, ix->tuning, ctx.num_sms, s, nullptr, launch_need(ix, q));
     if ((e = cudaGetLastError())) return cuda_fail(e, "match launch");
     if ((e = cudaMemcpyAsync(ix->host_err, w.ctr + kCtrError, 4, cudaMemcpyDeviceToHost, s))) return cuda_fail(e, "error word");
     if ((e = cudaMemcpyAsync(out_ids, w.out_ids, sumk * 4, cudaMemcpyDeviceToHost, s))) return cuda_fail(e, "result ids");
@@ -342,6 +356,8 @@ genie_index::~genie_index() {
     d_dir_row_key.release();
     d_bm_slot.release();
     d_bm_rows.release();
+    d_planes.release();
+    d_pl_vals.release();
     for (auto &d : dirs) {
         d.second->release();
         delete d.second;

@@ -42,9 +42,12 @@ struct Workspace {
     DevBuf out_ids, out_counts, out_scores;
     DevBuf counters;                 // per-object counters of a subsequence search
     DevBuf unit_key;
+    DevBuf planes;                   // per-query state of k_planes: bounds, histograms, key counts
     bool done_zeroed = false;
     int64_t done_q = 0;
     cudaError_t reserve(int64_t Q, int64_t items, int64_t units, int64_t sumk);
+    // what a search with an index's planes needs beside; before view()
+    cudaError_t reserve_planes(int64_t Q);
     void release();
     Work view(int64_t Q, bool scores) const;
 };
@@ -54,6 +57,13 @@ int validate_queries(const genie_queries *q, std::vector<int64_t> &out_off, int6
 // The device view of an index for a tuning: ix->dev plus the tile
 // directories of the tuning's two tile sizes (built on first use).
 DevIndex index_view(genie_index *ix, const Tuning &t);
+// Called with every batch of queries before it is searched: builds the
+// cumulative planes of a byte-valued index (planes.cu) once its searches are
+// worth them.
+void note_search(genie_index *ix, const genie_queries *q);
+// Kernels that a batch may need on an index with planes (LaunchNeed); a batch
+// without them needs kNeedLists.
+uint32_t launch_need(const genie_index *ix, const genie_queries *q);
 
 // Asynchronous steps of one batch for the serving loop (batch.cu): stage,
 // launch and download on the batch's own stream; poll; copy the results out.
@@ -104,6 +114,10 @@ struct genie_index {
     int64_t bm_words = 0;
     gg::DevBuf d_bm_slot, d_bm_rows;
     std::vector<std::pair<int32_t, gg::DevBuf *>> dirs;
+    int64_t pl_bytes = -1;           // what the planes take (0: the index has none, -1: not looked at)
+    int64_t pl_touched = 0;          // posting ids its searches have touched before they were built
+    int64_t pl_tiles = 0, pl_row_vec = 0;      // set once built
+    gg::DevBuf d_planes, d_pl_vals;
     cudaStream_t stream = nullptr;
     std::mutex mu;                   // serialises searches on this handle's workspace
     gg::Workspace ws;

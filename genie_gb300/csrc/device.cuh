@@ -28,6 +28,26 @@ enum : uint8_t { kFlagWeighted = 1, kFlagSmallCount = 2, kFlagRetry = 4, kFlagPa
 constexpr uint32_t kBmSpanCap = 1024;
 // posting ids of a query on the bitmap path (its 32-id chunk entries)
 constexpr uint32_t kBmMaxIds = 40 * 1024;
+// objects of one tile of the cumulative planes, items of a query counted with
+// them (eight count planes), and the largest k of a weighted query there (its
+// kept keys and as many new ones fit the candidate buffer)
+constexpr uint32_t kPlTile = 16384;
+constexpr uint32_t kPlMaxItems = 255;
+constexpr uint32_t kPlMaxWeightedK = 512;
+// weighted queries there: items up to which a weight group is 8 (else 16), the
+// largest unit weight, and the largest bound (eleven planes)
+constexpr uint32_t kPlGroup8 = 72;
+constexpr uint32_t kPlUnitMax = 31;
+constexpr uint32_t kPlBoundMax = 2047;
+// Whether a query of an index with planes is counted with them: m items that
+// end at item_end, counts of at most eight bits (one value per object and dim:
+// at most m), weighted results that fit a tile's buffer.  The plan decides by
+// it on the device, and the host by the same rule which kernels to launch.
+__host__ __device__ inline bool planes_take(int64_t m, int64_t item_end, bool weighted, uint32_t k, int32_t n_dims) {
+    return m <= (int64_t)kPlMaxItems && item_end <= 0xFFFFFFFFll && (!weighted || (k <= kPlMaxWeightedK && n_dims <= 65536));
+}
+// rows of a tile behind its keys' rows: no object, and every object
+constexpr uint32_t kPlExtraRows = 2;
 // zero bytes behind the posting ids of a plain index: 32 ids read from the
 // last position stay inside the allocation
 constexpr size_t kIdsPadBytes = 128;
@@ -69,6 +89,16 @@ struct DevIndex {
     const uint32_t *bm_slot;
     const uint32_t *bm_rows;
     int64_t bm_words;
+    // cumulative presence planes of a byte-valued index (planes.cu): in every
+    // tile of kPlTile objects, one row of pl_row_vec 16-byte vectors per key,
+    // then an empty and a full row.  Null when absent.
+    const uint4 *planes;
+    int64_t pl_tile_vec;           // vectors of a tile: (pl_keys + kPlExtraRows) * pl_row_vec
+    int64_t pl_keys;
+    const uint8_t *pl_vals;        // the values themselves, object by object: value - dim_min
+    int32_t pl_val_row;            // bytes of an object's row
+    int64_t pl_tiles;
+    int32_t pl_row_vec;
 };
 
 struct DevQueries {
@@ -97,6 +127,7 @@ struct QInfo {
     int32_t n_items;
     uint32_t k;
     int32_t scale;      // fixed-point exponent of a weighted query
+    int32_t qshift;     // k_planes, weighted: increments per unit of a tile's bounds, as a shift
     uint16_t parts;     // id-range parts
     uint8_t cls;        // kClsSparse / kClsDense / kClsNone
     uint8_t flags;
@@ -123,10 +154,12 @@ struct Tuning {
 
 // Work lists, one per kernel variant.
 enum : int { kListSparsePacked = 0, kListSparseWide = 1, kListDenseSmall = 2, kListDenseWide = 3,
-             kListBitmap = 4, kNumLists = 5 };
+             kListBitmap = 4, kListPlanes = 5, kListPlanesWeighted = 6, kNumLists = 7 };
 constexpr int kCtrError = 2 * kNumLists;     // ctr[2c] = items in list c, ctr[2c+1] = next
 constexpr int kCtrUnits = 2 * kNumLists + 2;  // 64-bit: units handed out to queries so far
-constexpr int kCtrWords = 2 * kNumLists + 4;
+constexpr int kCtrPlanes = 2 * kNumLists + 4;  // two 64-bit: (query, tile) pairs handed out per planes list
+constexpr int kCtrWords = 2 * kNumLists + 8;
+static_assert(kCtrUnits % 2 == 0 && kCtrPlanes % 2 == 0, "64-bit counters are aligned");
 
 // Device work state of one search (all arrays sized for the batch).
 struct Work {
@@ -146,6 +179,10 @@ struct Work {
     uint32_t *lb;          // [Q] lower bound on the k-th primary of a dense query (from its finished tiles)
     uint32_t *part_cnt;    // [Q*max_parts]
     uint64_t *scratch;     // [sum(k)*max_parts] part results (keys)
+    int64_t scratch_keys;  // keys the scratch holds
+    uint64_t *lbk;         // [Q] k_planes: lower bound on the query's final k-th key (null: no planes)
+    uint32_t *pl_cur;      // [Q] k_planes: keys its tiles have written
+    uint32_t *pl_hist;     // [Q*256] k_planes: their primaries (counts, or the top 8 of 31 bits)
     int32_t max_parts;     // parts of a dense query (<= kMaxDenseParts); scratch stride per result slot
     uint32_t *out_ids;
     uint32_t *out_counts;

@@ -61,6 +61,10 @@ __global__ void __launch_bounds__(kPlanThreads, 8) k_plan(DevIndex ix, DevQuerie
     __shared__ unsigned long long s_total, s_units, s_unit0;
     __shared__ unsigned int s_maxw, s_bad, s_multi, s_oob;
     __shared__ uint32_t s_tmp[48];
+    __shared__ uint32_t s_inc[kPlanThreads];       // planes, weighted: the items' increments
+    __shared__ unsigned long long s_groups;
+    __shared__ uint32_t s_top;
+    static_assert(kPlMaxItems < kPlanThreads, "one item of a planes query per thread");
     const int64_t q = blockIdx.x;
     const int64_t nq = Q.dyn ? (int64_t)Q.dyn[0] : (int64_t)Q.n_queries;
     if (q >= nq) return;
@@ -89,12 +93,21 @@ __global__ void __launch_bounds__(kPlanThreads, 8) k_plan(DevIndex ix, DevQuerie
     if (s_oob) return;
     const bool weighted = Q.weighted && Q.weight && Q.weighted[q];
     const bool exact = Q.dyn && Q.dyn[2];      // a batch of exact items sends no upper bounds
+    // Counted from the cumulative planes whenever the index has them: a range
+    // item costs two rows of 1/8 byte an object whatever it covers, against 4
+    // bytes and a shared atomic per posting id elsewhere.  Even exact items
+    // (1 % of the objects each) are faster there than hashed: 260,000 x 128,
+    // 256 queries of 8-128 items, a quarter of them exact, 494 us before (125
+    // of them hashing the exact ones) and 140 us.
+    const bool planes = ix.planes != nullptr && W.lbk != nullptr && planes_take(m, i1, weighted, k, ix.n_dims);
     if (tid == 0) {
         s_total = 0;
         s_units = 0;
         s_maxw = 0;
         s_bad = 0;
         s_multi = 0;
+        s_groups = 0;
+        s_top = 0;
     }
     __syncthreads();
     int32_t scale = 0;
@@ -121,6 +134,10 @@ __global__ void __launch_bounds__(kPlanThreads, 8) k_plan(DevIndex ix, DevQuerie
     uint64_t total = 0, units = 0;
     int64_t k0_first = 0, a_first = 0, e_first = 0;     // a, e: list offsets around the keys
     uint32_t nk_first = 0, inc_first = 1;
+    // planes of low - 1 and up of this thread's item (byte offsets in a tile)
+    const uint32_t pl_row = planes ? (uint32_t)ix.pl_row_vec * 16u : 0u;
+    uint32_t test = 0;       // its dim, low and width, low relative to the dim's least value
+    uint2 rows = make_uint2((uint32_t)ix.pl_keys * pl_row, ((uint32_t)ix.pl_keys + 1u) * pl_row);
     for (int64_t i = i0 + tid; i < i1; i += nt) {
         if (!GG_OK(i, W.items_cap, 7)) break;
         int32_t d = Q.dim[i], lo = Q.low[i], hi = exact ? lo : Q.up[i];
@@ -135,6 +152,11 @@ __global__ void __launch_bounds__(kPlanThreads, 8) k_plan(DevIndex ix, DevQuerie
                 a = ix.key_off[k0];
                 e = ix.key_off[k0 + nk];
                 total += (uint64_t)(e - a);
+                if (planes) {
+                    if (lo > mn) rows.x = (uint32_t)(k0 - 1) * pl_row;
+                    if (hi < mx) rows.y = (uint32_t)(k0 + nk - 1) * pl_row;
+                    test = (uint32_t)d << 16 | (uint32_t)(lo - mn) << 8 | (uint32_t)(hi - lo);
+                }
             }
         }
         uint32_t inc = 1;
@@ -143,7 +165,7 @@ __global__ void __launch_bounds__(kPlanThreads, 8) k_plan(DevIndex ix, DevQuerie
         // of the query is, the query's units are its items and nothing more
         // is written.  Otherwise the query takes a unit range past the
         // batch's items and these slots, in its own item range, stay unread.
-        if (nk <= 1 && i < W.units_cap) {
+        if (nk <= 1 && i < W.units_cap && !planes) {
             if (ix.codec) {
                 a = nk ? ix.key_seg[k0] : 0;
                 e = nk ? ix.key_seg[k0 + 1] : 0;
@@ -185,7 +207,7 @@ __global__ void __launch_bounds__(kPlanThreads, 8) k_plan(DevIndex ix, DevQuerie
     const bool fits = unit0 + n_units <= W.units_cap;
     if (tid == 0 && !fits) atomicOr(&W.ctr[kCtrError], kErrUnits);
     // one unit per covered list (a query with several lists in one item)
-    if (fits && !single) {
+    if (fits && !single && !planes) {
         int64_t base = unit0;
         for (int64_t c = i0; c < i1; c += nt) {
             const int64_t i = c + tid;
@@ -230,6 +252,44 @@ __global__ void __launch_bounds__(kPlanThreads, 8) k_plan(DevIndex ix, DevQuerie
     qi.total = (int64_t)total;
     qi.unit0 = unit0;
     qi.n_units = (int32_t)n_units;
+    qi.qshift = 0;
+    if (planes && fits) {
+        // the items that can match, as plane rows in the query's item slots;
+        // by descending weight when weighted, with the unit of the tiles'
+        // bounds: the groups' largest weights, rounded up, within eleven bits
+        const int64_t i = i0 + tid;
+        const bool live = i < i1 && nk_first > 0 && inc_first > 0;
+        qi.unit0 = i0;
+        qi.n_units = __syncthreads_count(live);
+        uint32_t at = 0;
+        if (!weighted) {
+            at = block_excl_scan(live ? 1u : 0u, s_tmp, nullptr);
+        } else {
+            s_inc[tid] = live ? inc_first : 0u;
+            __syncthreads();
+            for (int32_t j = 0; j < m; ++j)
+                at += (s_inc[j] > inc_first || (s_inc[j] == inc_first && j < (int32_t)tid)) ? 1u : 0u;
+            const uint32_t group = (uint32_t)qi.n_units <= kPlGroup8 ? 8u : 16u;
+            if (live && at % group == 0) atomicAdd(&s_groups, (unsigned long long)group * inc_first);
+            if (live && at == 0) s_top = inc_first;
+            __syncthreads();
+            // every group rounds its unit weight up
+            const uint64_t up = (uint64_t)group * (((uint32_t)qi.n_units + group - 1) / group);
+            while (qi.qshift < 31 && ((s_groups >> qi.qshift) + up > kPlBoundMax ||
+                                      ((uint64_t)s_top + ((1ull << qi.qshift) - 1)) >> qi.qshift > kPlUnitMax))
+                ++qi.qshift;
+        }
+        if (live && GG_OK(i0 + at, W.units_cap, 14)) {
+            *(uint2 *)&W.span_start[i0 + at] = rows;
+            W.inc[i0 + at] = inc_first;
+            W.item_nk[i0 + at] = test;
+        }
+        W.pl_hist[(size_t)q * 256 + tid] = 0;
+        if (tid == 0) {
+            W.lbk[q] = 0;
+            W.pl_cur[q] = 0;
+        }
+    }
     qi.item0 = i0;
     qi.n_items = m;
     qi.k = k;
@@ -254,7 +314,10 @@ __global__ void __launch_bounds__(kPlanThreads, 8) k_plan(DevIndex ix, DevQuerie
             const int64_t slots = packed ? T.sparse_slots_packed : T.sparse_slots_wide;
             const int64_t cap = slots * T.sparse_load_pct / 100;     // table load factor bound
             const int64_t ps = (total + cap - 1) / cap;
-            if (total <= T.sparse_max_total && total * 4 <= ix.n_objects * 3 && packed && !ix.codec &&
+            if (planes) {
+                qi.cls = kClsDense;
+                list = weighted ? kListPlanesWeighted : kListPlanes;
+            } else if (total <= T.sparse_max_total && total * 4 <= ix.n_objects * 3 && packed && !ix.codec &&
                 T.bitmap_bits > 0 && T.bitmap_ready && ix.n_objects <= T.bitmap_bits &&
                 qi.n_units <= (int32_t)kBmSpanCap && total <= (int64_t)kBmMaxIds &&
                 ix.n_ids <= (int64_t)0xFFFFFFFFll - 64) {       // posting positions in 32 bits
@@ -276,12 +339,17 @@ __global__ void __launch_bounds__(kPlanThreads, 8) k_plan(DevIndex ix, DevQuerie
         }
         W.qinfo[q] = qi;
         if (list >= 0) {
-            // a dense list holds the query once: its parts are taken part-major
-            const uint32_t entries = (list == kListDenseSmall || list == kListDenseWide) ? 1u : qi.parts;
+            // a dense or planes list holds the query once: its parts (tiles) are taken part-major
+            const uint32_t entries = qi.cls == kClsDense ? 1u : qi.parts;
             uint2 *wl = W.work + (size_t)list * W.work_stride;
             uint32_t b = atomicAdd(&W.ctr[2 * list], entries);
-            for (uint32_t p = 0; p < entries; ++p)
-                if (GG_OK(b + p, W.work_stride, 8)) wl[b + p] = make_uint2((uint32_t)q, p);
+            if (planes) {      // what a tile needs to start: query, item slots, items | k, unit shift
+                if (GG_OK(2 * b + 1, W.work_stride, 8))
+                    ((uint4 *)wl)[b] = make_uint4((uint32_t)q, (uint32_t)i0, (uint32_t)qi.n_units | k << 16, (uint32_t)qi.qshift);
+            } else {
+                for (uint32_t p = 0; p < entries; ++p)
+                    if (GG_OK(b + p, W.work_stride, 8)) wl[b + p] = make_uint2((uint32_t)q, p);
+            }
         }
     }
     // queries without any matching posting: padded results right away
@@ -999,6 +1067,7 @@ __global__ void __launch_bounds__(NT, NT == 512 ? 2 : 1) k_sparse(DevIndex ix, D
 }  // namespace gg
 
 #include "bitmap.cuh"
+#include "planes.cuh"
 
 namespace gg {
 
@@ -1494,6 +1563,26 @@ int launch_plan(const DevIndex &ix, const DevQueries &Q, const Work &W, const Tu
 // The match kernels as persistent grids: the bitmap kernel, the sparse
 // kernel (both slot widths), the dense kernel (both counter widths).
 enum : int { kKernBitmap = 0, kKernSparse = 1, kKernDense = 2, kNumKern = 3 };
+
+// The planes kernels of a byte-valued index: the tiles of unweighted queries,
+// those of weighted ones, and the merge of both.
+int launch_planes(const DevIndex &ix, const DevQueries &Q, const Work &W, int num_sms, cudaStream_t s, uint32_t need) {
+    if (!ix.planes || !W.lbk) return 0;
+    int n = 0;
+    if (need & kNeedPlanes) {
+        k_planes<false><<<num_sms * PlConfig<false>::kBlocks, kPlThreads, 0, s>>>(ix, Q, W);
+        ++n;
+    }
+    if (need & kNeedPlanesWeighted) {
+        k_planes<true><<<num_sms * PlConfig<true>::kBlocks, kPlThreads, 0, s>>>(ix, Q, W);
+        ++n;
+    }
+    if (n && ix.pl_tiles > 1) {
+        k_planes_finish<<<num_sms * 2, kPlThreads, 0, s>>>(ix, Q, W);
+        ++n;
+    }
+    return n;
+}
 int launch_kernel(int kern, const DevIndex &ix, const DevQueries &Q, const Work &W, const Tuning &t, int num_sms,
                   cudaStream_t s) {
     // persistent grids: as many CTAs as fit on every SM at once
@@ -1524,8 +1613,9 @@ int launch_kernel(int kern, const DevIndex &ix, const DevQueries &Q, const Work 
 }
 
 int launch_match(const DevIndex &ix, const DevQueries &Q, const Work &W, const Tuning &tun,
-                 int num_sms, cudaStream_t s, cudaEvent_t *ev) {
+                 int num_sms, cudaStream_t s, cudaEvent_t *ev, uint32_t need) {
     if (Q.n_queries <= 0) return 0;
+    if (!ix.planes || !W.lbk) need = kNeedLists;
     const Tuning t = launch_tuning(ix, tun, num_sms);
     int launches = 0;
     if (ev) cudaEventRecord(ev[0], s);
@@ -1533,7 +1623,8 @@ int launch_match(const DevIndex &ix, const DevQueries &Q, const Work &W, const T
     if (ev) cudaEventRecord(ev[1], s);
     // dense last: sparse parts that overflow are re-queued to the dense lists
     for (int k = 0; k < kNumKern; ++k) {
-        launches += launch_kernel(k, ix, Q, W, t, num_sms, s);
+        if (k == kKernDense) launches += launch_planes(ix, Q, W, num_sms, s, need);
+        if (need & kNeedLists) launches += launch_kernel(k, ix, Q, W, t, num_sms, s);
         if (ev) cudaEventRecord(ev[2 + k], s);
     }
     return launches;

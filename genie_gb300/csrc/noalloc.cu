@@ -130,6 +130,10 @@ extern "C" int genie_search_noalloc(genie_index *ix, const genie_queries *q, con
     w.lb = (uint32_t *)(base + kNa.lb);
     w.part_cnt = (uint32_t *)(base + kNa.part_cnt);
     w.scratch = (uint64_t *)(base + kNa.scratch);
+    w.scratch_keys = kNaMaxResults * kMaxParts;
+    w.lbk = nullptr;              // no planes: ix->dev holds none
+    w.pl_cur = nullptr;
+    w.pl_hist = nullptr;
     w.max_parts = kMaxParts;      // the fixed array holds 16 part results per result slot
     w.out_ids = out_ids;
     w.out_counts = out_counts;

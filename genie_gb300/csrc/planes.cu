@@ -1,0 +1,223 @@
+// planes.cu -- cumulative presence planes of a byte-valued index.
+//
+// For every (dim, value) of a table whose dims span at most 256 values, one
+// bit per object: set when the object's value on that dim is at most the
+// list's value.  An item [low, up] matches plane(up) & ~plane(low - 1), so a
+// range costs two rows however many lists it covers (planes.cuh counts with
+// them).  A plane row is n_objects / 8 bytes against 4 bytes a posting id, so
+// the planes take (values per dim) / 32 times the ids' bytes: eight times for
+// 256 values.  They are built when a quarter of the device memory that is free
+// then holds them, once per index (note_search), and kept while it lives.  The
+// values themselves are kept too, one byte each, object by object (a 32nd of
+// 256 planes): a weighted tile sums its few candidates from them, whose bytes
+// of one object lie in one or two lines, where the planes would cost a line
+// per item and candidate.
+//
+// Layout: tile by tile (kPlTile objects), in a tile one row of 16-byte vectors
+// per key, so the rows that run together lie together (few pages at a time,
+// and one tile's used rows fit L2), then an empty and a full row for the open
+// ends.  The row of a dim's largest value (every object) is never read and not
+// written.  Offsets in a tile are 32-bit bytes.
+#include "capi_internal.h"
+
+#include <algorithm>
+
+namespace gg {
+namespace {
+
+constexpr int64_t kPlMaxValues = 256;
+constexpr int kPlSubWords = 64;                          // words of a row one CTA builds (2,048 objects)
+constexpr int kPlBuildThreads = 256;
+constexpr size_t kPlColumnBytes = size_t(512) << 20;     // column bytes held at a time
+
+// col[d][id] = value - dim_min of every object on dims [d0, d0 + nd), from
+// the posting lists (one list per blockIdx.x, slices in blockIdx.y).
+__global__ void k_pl_columns(const uint32_t *__restrict__ ids, const int64_t *__restrict__ key_off,
+                             const int64_t *__restrict__ key_base, int32_t d0, int32_t nd, int64_t n,
+                             uint8_t *__restrict__ col) {
+    const int64_t key = key_base[d0] + blockIdx.x;
+    int32_t lo = 0, hi = nd - 1;                // the dim holding the key
+    while (lo < hi) {
+        const int32_t mid = (lo + hi + 1) >> 1;
+        if (key_base[d0 + mid] <= key) lo = mid; else hi = mid - 1;
+    }
+    const uint8_t v = (uint8_t)(key - key_base[d0 + lo]);
+    uint8_t *c = col + (int64_t)lo * n;
+    const int64_t a = key_off[key], e = key_off[key + 1];
+    for (int64_t p = a + (int64_t)blockIdx.y * blockDim.x + threadIdx.x; p < e; p += (int64_t)gridDim.y * blockDim.x)
+        c[ids[p]] = v;
+}
+
+// One dim (blockIdx.y) of kPlSubWords * 32 objects (blockIdx.x): presence bits
+// per value in shared memory, an OR over the values in order, rows out.  Four
+// threads share a word's values, so the running OR takes two passes.
+__global__ void __launch_bounds__(kPlBuildThreads) k_pl_build(const uint8_t *__restrict__ col,
+                                                              const int64_t *__restrict__ key_base, int32_t d0,
+                                                              int64_t n, int64_t tile_words, uint32_t row_words,
+                                                              uint32_t subs, uint32_t *__restrict__ planes) {
+    extern __shared__ uint32_t eq[];           // [values][kPlSubWords]
+    __shared__ uint32_t part[4][kPlSubWords];
+    const int32_t d = d0 + blockIdx.y;
+    const uint32_t values = (uint32_t)(key_base[d + 1] - key_base[d]);
+    const uint64_t tile = blockIdx.x / subs;
+    const uint32_t sub = (uint32_t)(blockIdx.x % subs);
+    const int64_t o0 = (int64_t)tile * kPlTile + (int64_t)sub * kPlSubWords * 32;
+    for (uint32_t i = threadIdx.x; i < values * kPlSubWords; i += kPlBuildThreads) eq[i] = 0;
+    __syncthreads();
+    const uint8_t *c = col + (int64_t)blockIdx.y * n;
+    for (int64_t i = threadIdx.x; i < kPlSubWords * 32; i += kPlBuildThreads)
+        if (o0 + i < n) atomicOr(&eq[(uint32_t)c[o0 + i] * kPlSubWords + (uint32_t)(i >> 5)], 1u << (i & 31));
+    __syncthreads();
+    const uint32_t w = threadIdx.x % kPlSubWords, seg = threadIdx.x / kPlSubWords;
+    const uint32_t per = (values + 3) / 4;
+    const uint32_t v0 = min(values, seg * per), v1 = min(values, v0 + per);
+    uint32_t acc = 0;
+    for (uint32_t v = v0; v < v1; ++v) {
+        acc |= eq[v * kPlSubWords + w];
+        eq[v * kPlSubWords + w] = acc;
+    }
+    part[seg][w] = acc;
+    __syncthreads();
+    uint32_t before = 0;
+    for (uint32_t g = 0; g < seg; ++g) before |= part[g][w];
+    const uint32_t word = sub * kPlSubWords + w;
+    if (word >= row_words) return;
+    uint32_t *out = planes + tile * (uint64_t)tile_words + (uint64_t)key_base[d] * row_words + word;
+    for (uint32_t v = v0; v < v1 && v + 1 < values; ++v) out[(uint64_t)v * row_words] = eq[v * kPlSubWords + w] | before;
+}
+
+// The columns of dims [d0, d0 + nd) into the objects' rows (32 x 32 tiles through shared memory).
+__global__ void k_pl_rows(const uint8_t *__restrict__ col, int32_t d0, int32_t nd, int64_t n, int32_t row,
+                          uint8_t *__restrict__ vals) {
+    __shared__ uint8_t tile[32][33];
+    const int64_t o0 = (int64_t)blockIdx.x * 32;
+    const int32_t c0 = (int32_t)blockIdx.y * 32;
+    for (int y = threadIdx.y; y < 32; y += blockDim.y)
+        if (c0 + y < nd && o0 + threadIdx.x < n) tile[y][threadIdx.x] = col[(int64_t)(c0 + y) * n + o0 + threadIdx.x];
+    __syncthreads();
+    for (int y = threadIdx.y; y < 32; y += blockDim.y)
+        if (o0 + y < n && c0 + (int)threadIdx.x < nd) vals[(o0 + y) * row + d0 + c0 + threadIdx.x] = tile[threadIdx.x][y];
+}
+
+// The empty and the full row behind each tile's keys.
+__global__ void k_pl_ends(uint4 *planes, int64_t tiles, int64_t keys, int64_t row_vec) {
+    for (int64_t t = blockIdx.x; t < tiles; t += gridDim.x) {
+        uint4 *r = planes + (t * (keys + kPlExtraRows) + keys) * row_vec;
+        for (int64_t i = threadIdx.x; i < row_vec; i += blockDim.x) {
+            r[i] = make_uint4(0, 0, 0, 0);
+            r[row_vec + i] = make_uint4(0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu);
+        }
+    }
+}
+
+// Bytes of the index's planes; 0 when it has none.
+int64_t planes_bytes(const genie_index *ix) {
+    const HostIndex &h = ix->host;
+    const int64_t n = h.n_objects, nk = h.n_keys();
+    if (ix->is_bag || ix->sub_shift >= 0 || ix->codec || n <= 0 || nk <= 0) return 0;
+    for (int32_t j = 0; j < h.n_dims; ++j)
+        if (h.key_base[j + 1] - h.key_base[j] > kPlMaxValues) return 0;
+    const int64_t tiles = (n + kPlTile - 1) / kPlTile;
+    const int64_t row_vec = tiles > 1 ? (int64_t)kPlTile / 128 : (n + 127) / 128, rows = nk + kPlExtraRows;
+    if (rows * row_vec * 16 > (int64_t)0xFFFFFFFFll || tiles > (int64_t)0x7FFFFFFF) return 0;
+    return tiles * rows * row_vec * 16;
+}
+
+bool build(genie_index *ix) {
+    const HostIndex &h = ix->host;
+    const int64_t n = h.n_objects, nk = h.n_keys();
+    const int64_t tiles = (n + kPlTile - 1) / kPlTile;
+    const int64_t row_vec = tiles > 1 ? (int64_t)kPlTile / 128 : (n + 127) / 128, rows = nk + kPlExtraRows;
+    const size_t bytes = (size_t)ix->pl_bytes;
+    const int32_t dims_at_once = (int32_t)std::min<int64_t>(h.n_dims, std::max<int64_t>(1, (int64_t)kPlColumnBytes / n));
+    const int32_t val_row = (h.n_dims + 15) & ~15;
+    size_t free_b = 0, total_b = 0;
+    if (cudaMemGetInfo(&free_b, &total_b)) {
+        cudaGetLastError();
+        return false;
+    }
+    if (bytes > free_b / 4) return false;
+    static_assert(kPlMaxValues * kPlSubWords * 4 == 65536, "shared presence bits");
+    DevBuf col;
+    cudaError_t e;
+    if ((e = cudaFuncSetAttribute((const void *)k_pl_build, cudaFuncAttributeMaxDynamicSharedMemorySize, 65536)) ||
+        (e = cudaMalloc(&ix->d_planes.p, bytes)) ||
+        (e = ix->d_pl_vals.reserve((size_t)n * (size_t)val_row)) || (e = cudaMalloc(&col.p, (size_t)dims_at_once * (size_t)n))) {
+        cudaGetLastError();
+        ix->d_planes.release();
+        ix->d_pl_vals.release();
+        return false;
+    }
+    ix->d_planes.bytes = bytes;
+    const uint32_t subs = (uint32_t)((row_vec * 4 + kPlSubWords - 1) / kPlSubWords);
+    const unsigned slices = (unsigned)std::min<int64_t>(64, std::max<int64_t>(1, n / 65536));
+    for (int32_t d0 = 0; d0 < h.n_dims; d0 += dims_at_once) {
+        const int32_t nd = std::min(dims_at_once, h.n_dims - d0);
+        const unsigned keys = (unsigned)(h.key_base[d0 + nd] - h.key_base[d0]);
+        int64_t widest = 1;
+        for (int32_t j = d0; j < d0 + nd; ++j) widest = std::max(widest, h.key_base[j + 1] - h.key_base[j]);
+        k_pl_columns<<<dim3(keys, slices), 256, 0, ix->stream>>>(ix->dev.ids, ix->dev.key_off, ix->dev.key_base, d0, nd,
+                                                                 n, (uint8_t *)col.p);
+        for (int32_t j = 0; j < nd; j += 32 * 65535)
+            k_pl_rows<<<dim3((unsigned)((n + 31) / 32), (unsigned)((std::min(nd - j, 32 * 65535) + 31) / 32)), dim3(32, 8), 0,
+                        ix->stream>>>((const uint8_t *)col.p + (int64_t)j * n, d0 + j, nd - j, n, val_row,
+                                      (uint8_t *)ix->d_pl_vals.p);
+        // grid y is at most 65,535 dims at once
+        for (int32_t j = 0; j < nd; j += 65535)
+            k_pl_build<<<dim3((unsigned)(tiles * subs), (unsigned)std::min(65535, nd - j)), kPlBuildThreads,
+                         (size_t)widest * kPlSubWords * 4, ix->stream>>>(
+                (const uint8_t *)col.p + (int64_t)j * n, ix->dev.key_base, d0 + j, n, rows * row_vec * 4,
+                (uint32_t)(row_vec * 4), subs, (uint32_t *)ix->d_planes.p);
+    }
+    k_pl_ends<<<(unsigned)std::min<int64_t>(tiles, 65535), 128, 0, ix->stream>>>((uint4 *)ix->d_planes.p, tiles, nk,
+                                                                                row_vec);
+    e = cudaGetLastError();
+    if (!e) e = cudaStreamSynchronize(ix->stream);
+    cudaFree(col.p);
+    if (e) {
+        cudaGetLastError();
+        ix->d_planes.release();
+        ix->d_pl_vals.release();
+        return false;
+    }
+    ix->pl_row_vec = row_vec;
+    ix->pl_tiles = tiles;
+    return true;
+}
+
+}  // namespace
+
+// Building the planes takes about as long as counting four times their bytes
+// of posting ids without them (260,000 x 128, 1.1 GB of planes: build 1 ms,
+// 2.5 GB of ids counted in 0.5 ms; 4,000,000 x 128, 17 GB: 13 ms, and 310 GB
+// in 45 ms), so they are built when the index's searches have touched that
+// much: a table searched once or twice never pays for them, and none pays more
+// than about twice what it would have.  Past that point nothing is counted.
+void note_search(genie_index *ix, const genie_queries *q) {
+    std::lock_guard<std::mutex> g(ix->dir_mu);
+    if (ix->pl_bytes < 0) ix->pl_bytes = planes_bytes(ix);
+    if (ix->pl_bytes == 0 || ix->pl_tiles > 0) return;
+    const HostIndex &h = ix->host;
+    const int64_t enough = ix->pl_bytes;       // ids, of four bytes
+    const int64_t n = q->n_queries > 0 ? q->item_off[q->n_queries] : 0;
+    for (int64_t i = 0; i < n && ix->pl_touched < enough; ++i) {
+        int64_t a = 0, e = 0;
+        item_span(h, q->dim[i], q->low[i], q->up[i], a, e);
+        ix->pl_touched += e - a;
+    }
+    if (ix->pl_touched >= enough && !build(ix)) ix->pl_bytes = 0;
+}
+
+uint32_t launch_need(const genie_index *ix, const genie_queries *q) {
+    uint32_t need = 0;
+    for (int64_t i = 0; i < q->n_queries; ++i) {
+        const bool w = q->weighted && q->weight && q->weighted[i];
+        const uint32_t k = q->k ? q->k[i] : q->uniform_k;
+        const int64_t a = q->item_off[i], e = q->item_off[i + 1];
+        if (!planes_take(e - a, e, w, k, ix->host.n_dims)) need |= kNeedLists;
+        else need |= w ? kNeedPlanesWeighted : kNeedPlanes;
+    }
+    return need;
+}
+
+}  // namespace gg

@@ -236,6 +236,15 @@ DevIndex index_view(genie_index *ix, const Tuning &t) {
     d.bm_slot = bm ? (const uint32_t *)ix->d_bm_slot.p : nullptr;
     d.bm_rows = bm ? (const uint32_t *)ix->d_bm_rows.p : nullptr;
     d.bm_words = bm ? ix->bm_words : 0;
+    if (t.dense_bitmaps && ix->pl_tiles > 0) {
+        d.planes = (const uint4 *)ix->d_planes.p;
+        d.pl_row_vec = (int32_t)ix->pl_row_vec;
+        d.pl_keys = ix->host.n_keys();
+        d.pl_tile_vec = (d.pl_keys + kPlExtraRows) * ix->pl_row_vec;
+        d.pl_tiles = ix->pl_tiles;
+        d.pl_vals = (const uint8_t *)ix->d_pl_vals.p;
+        d.pl_val_row = (ix->host.n_dims + 15) & ~15;
+    }
     return d;
 }
 
