@@ -38,53 +38,54 @@ struct Emitter {
     V &visit;
     __device__ Emitter(int d, V &v) : deltas(d), visit(v) {}
     __device__ __forceinline__ void emit(const uint32_t *val, int cnt) {
+        uint32_t v[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) v[j] = j < cnt ? val[j] : 0u;
+        emit_mask(v, (1u << cnt) - 1u);
+    }
+    // the same for the values j with bit j of `has` set (the others are 0): in
+    // a lane they keep their order, without being moved together
+    __device__ __forceinline__ void emit_mask(const uint32_t (&val)[4], uint32_t has) {
         // sequence position of this lane's first value (skipped when the
         // visitor does not use positions)
         uint32_t pos0 = 0;
         if (POS) {
-            const uint32_t cincl = warp_incl_scan((uint32_t)cnt);
-            pos0 = emitted + cincl - (uint32_t)cnt;
+            const uint32_t cnt = __popc(has), cincl = warp_incl_scan(cnt);
+            pos0 = emitted + cincl - cnt;
             emitted += __shfl_sync(0xffffffffu, cincl, 31);
         }
-        // stage 1: inclusive running sum within the lane, then across lanes
-        uint32_t loc[4];
-        uint32_t s = 0;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            if (j < cnt) s += val[j];
-            loc[j] = s;
-        }
-        if (deltas == 0) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-                if (j < cnt) visit(val[j], pos0 + j);
-            return;
-        }
-        uint32_t incl = warp_incl_scan(s);
-        uint32_t pre = carry1 + incl - s;
-        carry1 += __shfl_sync(0xffffffffu, incl, 31);
-        uint32_t v1[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) v1[j] = pre + loc[j];
-        if (deltas == 1) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-                if (j < cnt) visit(v1[j], pos0 + j);
-            return;
-        }
-        // stage 2 (SERIAL_DELTA_DELTA)
-        uint32_t s2 = 0, loc2[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            if (j < cnt) s2 += v1[j];
-            loc2[j] = s2;
-        }
-        uint32_t incl2 = warp_incl_scan(s2);
-        uint32_t pre2 = carry2 + incl2 - s2;
-        carry2 += __shfl_sync(0xffffffffu, incl2, 31);
+        uint32_t v[4] = {val[0], val[1], val[2], val[3]};
+        delta(v, has);
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-            if (j < cnt) visit(pre2 + loc2[j], pos0 + j);
+            if ((has >> j) & 1u) visit(v[j], pos0 + __popc(has & ((1u << j) - 1u)));
+    }
+    // a whole block, four values in every lane; the visitor takes a lane's four at once
+    __device__ __forceinline__ void emit_block(uint32_t (&v)[4]) {
+        delta(v);
+        visit.four(v, emitted + 4u * lane_id());
+        emitted += 128;
+    }
+    // running sums over the lane's values, then across lanes; absent values
+    // are 0 and their sums unused, and before the second stage
+    // (SERIAL_DELTA_DELTA) 0 again
+    __device__ __forceinline__ void delta(uint32_t (&v)[4], uint32_t has = 15u) {
+        if (deltas == 0) return;
+        sum(v, carry1);
+        if (deltas == 1) return;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) v[j] = (has >> j) & 1u ? v[j] : 0u;
+        sum(v, carry2);
+    }
+    __device__ __forceinline__ void sum(uint32_t (&v)[4], uint32_t &carry) {
+        v[1] += v[0];
+        v[2] += v[1];
+        v[3] += v[2];
+        const uint32_t incl = warp_incl_scan(v[3]);
+        const uint32_t pre = carry + incl - v[3];
+        carry += __shfl_sync(0xffffffffu, incl, 31);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) v[j] += pre;
     }
 };
 
@@ -109,6 +110,14 @@ struct RegWords {         // a segment of <= 64 words held two per lane
         const uint32_t x = word(i);      // every lane shuffles
         return cond ? x : 0u;
     }
+};
+
+struct SmemWords {        // a segment staged in shared memory; positions past it read its last word
+    const uint32_t *s;
+    int64_t base;
+    uint32_t last;
+    __device__ __forceinline__ uint32_t word(int64_t i) const { return s[min((uint32_t)(i - base), last)]; }
+    __device__ __forceinline__ uint32_t word_if(int64_t i, bool cond) const { return cond ? word(i) : 0u; }
 };
 
 // Words [w0, w1) as values, 32 per step.
@@ -164,6 +173,42 @@ __device__ __forceinline__ int64_t dec_bp32(const S &src, int64_t w0, E &em) {
     return p;
 }
 
+// The same from shared memory: a value is cut from its two words by one funnel
+// shift, unconditionally (a width of 0 masks everything away; bits past the
+// value's own are masked).
+template <class E>
+__device__ __forceinline__ int64_t dec_bp32(const SmemWords &src, int64_t w0, E &em) {
+    const uint32_t lane = lane_id(), mb = lane >> 3;
+    const uint32_t n = src.word(w0);
+    uint32_t p = (uint32_t)(w0 + 1 - src.base);
+    for (uint32_t done = 0; done < n && p <= src.last; done += 128) {
+        const uint32_t hdr = src.s[p];
+        const uint32_t rem = n - done;
+        const uint32_t used = rem >= 97 ? hdr : hdr & ~(0xFFFFFFFFu >> (8u * ((rem + 31) / 32)));
+        const uint32_t b = (used >> (24u - 8u * mb)) & 255u;
+        // words of the miniblocks before this lane's: the header's higher bytes
+        const uint32_t over = mb ? used >> (32u - 8u * mb) : 0u;
+        const uint32_t before = (over & 255u) + ((over >> 8) & 255u) + (over >> 16);
+        // every word a value touches lies before p + 1 + all (or, masked away, on it)
+        const uint32_t all = (used & 255u) + ((used >> 8) & 255u) + ((used >> 16) & 255u) + (used >> 24);
+        if (p + all > src.last) break;
+        const uint32_t mask = b >= 32 ? 0xFFFFFFFFu : (1u << b) - 1u;
+        const uint32_t *at = src.s + p + 1 + before;
+        uint32_t bit = (lane & 7u) * 4u * b;
+        uint32_t v[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const uint32_t wi = bit >> 5;
+            v[k] = __funnelshift_r(at[wi], at[wi + 1], bit) & mask;
+            bit += b;
+        }
+        if (rem >= 128) em.emit_block(v);
+        else em.emit(v, (int)min(4u, rem > 4 * lane ? rem - 4 * lane : 0u));
+        p += 1 + all;
+    }
+    return src.base + p;
+}
+
 // Varint bytes of words [w0, w1): a lane owns one word; each byte with bit 7
 // set ends a value of at most five bytes, so a value spans at most this word
 // and the previous one.
@@ -179,28 +224,23 @@ __device__ __forceinline__ void dec_varint(const S &src, int64_t w0, int64_t w1,
         uint32_t prv = __shfl_up_sync(0xffffffffu, cur, 1);
         if (lane == 0) prv = have_prev ? prev_last : 0u;
         const bool prv_valid = lane > 0 || have_prev;
-        // terminal flags of the 8-byte window [prv | cur]
-        const uint64_t win = ((uint64_t)cur << 32) | prv;
-        uint32_t vals[4];
-        int cnt = 0;
+        // the window's bytes in order: seven bits each into the running value,
+        // which a terminal byte ends; before this word's bytes only the value
+        // that the previous word leaves open counts
+        uint32_t vals[4], has = 0, acc = 0, sh = 0;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int pos = 4 + j;                       // byte index in the window
-            const uint32_t byte = (uint32_t)(win >> (8 * pos)) & 255u;
-            if (!(byte & 0x80u)) continue;
-            // walk back to the byte after the previous terminal (<= 4 bytes)
-            int start = pos;
-            while (start > 0 && (pos - start) < 4) {
-                const uint32_t pb = (uint32_t)(win >> (8 * (start - 1))) & 255u;
-                if (pb & 0x80u) break;
-                if (start - 1 < 4 && !prv_valid) break;
-                --start;
+        for (int t = 0; t < 8; ++t) {
+            const uint32_t byte = ((t < 4 ? prv >> (8 * t) : cur >> (8 * (t - 4)))) & 255u;
+            acc |= sh < 32u ? (byte & 0x7Fu) << sh : 0u;
+            sh += 7;
+            if (t >= 4) vals[t - 4] = (byte & 0x80u) ? acc : 0u;
+            if ((byte & 0x80u) || (t == 3 && !prv_valid)) {
+                if (t >= 4) has |= 1u << (t - 4);
+                acc = 0;
+                sh = 0;
             }
-            uint32_t v = 0;
-            for (int t = pos; t >= start; --t) v = (v << 7) | ((uint32_t)(win >> (8 * t)) & 0x7Fu);
-            vals[cnt++] = v;
         }
-        em.emit(vals, cnt);
+        em.emit_mask(vals, has);
         prev_last = __shfl_sync(0xffffffffu, cur, 31);
         have_prev = true;
     }
@@ -236,17 +276,33 @@ __device__ __forceinline__ void decode_words(int codec, const S &src, int64_t w0
     }
 }
 
-// Decode one encoded segment and visit (value, sequence position) in order.
-// A segment of at most 64 words is read in one coalesced step and decoded
-// from registers; a longer one is read word by word.
+// Longest segment decoded from shared memory; the buffer holds two words more
+// (a value's second word may lie past the segment).
+constexpr uint32_t kStageWords = 1150;
+
+// Decode one encoded segment and visit (value, sequence position) in order,
+// and whole lanes of four by visit.four(values, position).  The segment's words
+// are first copied to shared memory in coalesced steps, so the chain of block
+// headers (each tells where the next one is) costs shared loads; a longer
+// segment is read word by word.
 template <class V>
 __device__ __forceinline__ void decode_segment(int codec, const uint32_t *__restrict__ w, int64_t w0, int64_t w1,
-                                               V &visit) {
-    if (w1 - w0 <= 64) {
-        const uint32_t lane = lane_id();
-        RegWords src{w0, w0 + lane < w1 ? __ldg(w + w0 + lane) : 0u,
-                     w0 + 32 + lane < w1 ? __ldg(w + w0 + 32 + lane) : 0u};
-        decode_words<true>(codec, src, w0, w1, visit);
+                                               uint32_t *stage, V &visit) {
+    if (w1 - w0 <= (int64_t)kStageWords) {
+        const uint32_t n = (uint32_t)(w1 - w0), lane = lane_id();
+        if (n == 0) return;
+        __syncwarp();
+        for (uint32_t b = 0; b < n; b += 32 * 8) {
+            uint32_t x[8];
+#pragma unroll
+            for (int r = 0; r < 8; ++r) x[r] = b + 32 * r + lane < n ? __ldg(w + w0 + b + 32 * r + lane) : 0u;
+#pragma unroll
+            for (int r = 0; r < 8; ++r)
+                if (b + 32 * r + lane < n) stage[b + 32 * r + lane] = x[r];
+        }
+        if (lane < 2) stage[n + lane] = 0;
+        __syncwarp();
+        decode_words<true>(codec, SmemWords{stage, w0, n - 1}, w0, w1, visit);
     } else {
         decode_words<true>(codec, GlobalWords{w}, w0, w1, visit);
     }
