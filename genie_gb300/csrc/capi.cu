@@ -66,17 +66,24 @@ DeviceContext &device_context(int dev) {
     return c;
 }
 
-cudaError_t Workspace::reserve(int64_t Q, int64_t items, int64_t units, int64_t sumk) {
+cudaError_t alloc_host_words(genie_index *ix) { return cudaMallocHost((void **)&ix->host_err, 256 + kCallBytes); }
+
+cudaError_t Workspace::reserve(int64_t Q, int64_t items, int64_t units, int64_t sumk, bool io) {
     cudaError_t e;
 #define RES(buf, n) if ((e = buf.reserve((size_t)(n))) != cudaSuccess) return e
-    RES(item_off, (Q + 1) * 8);
-    RES(dim, items * 4 + 16);
-    RES(low, items * 4 + 16);
-    RES(up, items * 4 + 16);
-    RES(weight, items * 4 + 16);
-    RES(weighted, Q + 16);
-    RES(k, Q * 4 + 16);
-    RES(out_off, (Q + 1) * 8);
+    if (io) {
+        RES(item_off, (Q + 1) * 8);
+        RES(dim, items * 4 + 16);
+        RES(low, items * 4 + 16);
+        RES(up, items * 4 + 16);
+        RES(weight, items * 4 + 16);
+        RES(weighted, Q + 16);
+        RES(k, Q * 4 + 16);
+        RES(out_off, (Q + 1) * 8);
+        RES(out_ids, sumk * 4 + 16);
+        RES(out_counts, sumk * 4 + 16);
+        RES(out_scores, sumk * 4 + 16);
+    }
     RES(item_k0, items * 8 + 16);
     RES(item_nk, items * 4 + 16);
     RES(item_inc, items * 4 + 16);
@@ -92,9 +99,6 @@ cudaError_t Workspace::reserve(int64_t Q, int64_t items, int64_t units, int64_t 
     RES(lb, Q * 4 + 16);
     RES(part_cnt, Q * kMaxDenseParts * 4 + 16);
     RES(scratch, sumk * kMaxDenseParts * 8 + 16);
-    RES(out_ids, sumk * 4 + 16);
-    RES(out_counts, sumk * 4 + 16);
-    RES(out_scores, sumk * 4 + 16);
 #undef RES
     if (!done_zeroed || done_q < Q) {
         cudaMemset(done.p, 0, done.bytes);
@@ -115,7 +119,7 @@ void Workspace::release() {
     DevBuf *all[] = {&item_off, &dim, &low, &up, &weight, &weighted, &k, &out_off, &item_k0, &item_nk,
                      &item_inc, &span_start,
                      &span_len, &inc, &qinfo, &work, &ctr, &qstate, &done, &lb, &part_cnt, &scratch,
-                     &out_ids, &out_counts, &out_scores, &counters, &unit_key, &planes};
+                     &out_ids, &out_counts, &out_scores, &counters, &unit_key, &call, &planes};
     for (DevBuf *b : all) b->release();
 }
 
@@ -291,6 +295,20 @@ int finish_loaded_index(genie_index *ix, genie_index **out) {
     return GENIE_OK;
 }
 
+// After a search's stream has been waited for: its error, and the results of a small call.
+int finish_search(genie_index *ix, uint32_t *out_ids, uint32_t *out_counts, float *out_scores) {
+    if (ix->call_results < 0) return check_device_error(*ix->host_err);
+    const unsigned char *ctr = (const unsigned char *)ix->host_err + 256 + ix->call_ctr;
+    const size_t n = (size_t)ix->call_results * 4, step = (n + 15) & ~(size_t)15;
+    const unsigned char *r = ctr + ((kCtrWords * 4 + 15) & ~15);
+    ix->call_results = -1;
+    if (int rc = check_device_error(((const uint32_t *)ctr)[kCtrError])) return rc;
+    memcpy(out_ids, r, n);
+    memcpy(out_counts, r + step, n);
+    if (out_scores) memcpy(out_scores, r + 2 * step, n);
+    return GENIE_OK;
+}
+
 int run_search(genie_index *ix, const genie_queries *q, const std::vector<int64_t> &out_off, int64_t n_items,
                uint32_t *out_ids, uint32_t *out_counts, float *out_scores, bool sync) {
     if (ix->sub_shift >= 0) return subseq_search(ix, q, out_off, n_items, out_ids, out_counts, out_scores, sync);
@@ -298,48 +316,108 @@ int run_search(genie_index *ix, const genie_queries *q, const std::vector<int64_
     const int64_t sumk = out_off[Q];
     note_search(ix, q);
     Workspace &ws = ix->ws;
-    cudaError_t e = ws.reserve(Q, n_items, count_units(ix->host, q), sumk);
+    const bool has_w = q->weighted && q->weight;
+    // A small call is packed: inputs and zeroed counters in one upload, error
+    // word and results in one download, both through pinned memory (a lookup in
+    // 1,000 x 128: 60 us with eight uploads from and three downloads to
+    // pageable memory and a memset, 42 us so).  A larger one is not: copying
+    // it once more on the host costs more than its copies do.
+    size_t at = 0;
+    auto place = [&](size_t n) {
+        const size_t o = at;
+        at += (n + 15) & ~(size_t)15;
+        return o;
+    };
+    const size_t o_item_off = place((size_t)(Q + 1) * 8), o_out_off = place((size_t)(Q + 1) * 8);
+    const size_t o_k = place(q->k ? (size_t)Q * 4 : 0), o_weighted = place(has_w ? (size_t)Q : 0);
+    const size_t o_dim = place((size_t)n_items * 4), o_low = place((size_t)n_items * 4);
+    const size_t o_up = q->up == q->low ? o_low : place((size_t)n_items * 4);
+    const size_t o_weight = place(has_w ? (size_t)n_items * 4 : 0);
+    const size_t o_ctr = place(kCtrWords * 4), up_bytes = at;
+    const size_t o_ids = place((size_t)sumk * 4), o_counts = place((size_t)sumk * 4);
+    const size_t o_scores = place(out_scores ? (size_t)sumk * 4 : 0);
+    const bool small = at <= kCallBytes && ix->host_err != nullptr;
+    cudaError_t e = ws.reserve(Q, n_items, count_units(ix->host, q), sumk, !small);
+    if (!e && small) e = ws.call.reserve(kCallBytes);
     if (e) return cuda_fail(e, "search workspace");
     cudaStream_t s = ix->stream;
-#define H2D(dst, src, n) if ((n) > 0 && (e = cudaMemcpyAsync(dst, src, (size_t)(n), cudaMemcpyHostToDevice, s))) return cuda_fail(e, "query upload")
-    H2D(ws.item_off.p, q->item_off, (Q + 1) * 8);
-    H2D(ws.dim.p, q->dim, n_items * 4);
-    H2D(ws.low.p, q->low, n_items * 4);
-    H2D(ws.up.p, q->up, n_items * 4);
-    const bool has_w = q->weighted && q->weight;
-    if (has_w) {
-        H2D(ws.weight.p, q->weight, n_items * 4);
-        H2D(ws.weighted.p, q->weighted, Q);
-    }
-    if (q->k) H2D(ws.k.p, q->k, Q * 4);
-    H2D(ws.out_off.p, out_off.data(), (Q + 1) * 8);
-#undef H2D
     DevQueries dq;
     dq.n_queries = (int32_t)Q;
-    dq.item_off = (const int64_t *)ws.item_off.p;
-    dq.dim = (const int32_t *)ws.dim.p;
-    dq.low = (const int32_t *)ws.low.p;
-    dq.up = (const int32_t *)ws.up.p;
-    dq.weight = has_w ? (const float *)ws.weight.p : nullptr;
-    dq.weighted = has_w ? (const uint8_t *)ws.weighted.p : nullptr;
-    dq.k = q->k ? (const uint32_t *)ws.k.p : nullptr;
     dq.uniform_k = q->uniform_k;
-    dq.out_off = (const int64_t *)ws.out_off.p;
     dq.dyn = nullptr;
+    unsigned char *dev = (unsigned char *)ws.call.p, *host = (unsigned char *)ix->host_err + 256;
+    if (small) {
+        memcpy(host + o_item_off, q->item_off, (size_t)(Q + 1) * 8);
+        memcpy(host + o_out_off, out_off.data(), (size_t)(Q + 1) * 8);
+        if (q->k) memcpy(host + o_k, q->k, (size_t)Q * 4);
+        memcpy(host + o_dim, q->dim, (size_t)n_items * 4);
+        memcpy(host + o_low, q->low, (size_t)n_items * 4);
+        if (o_up != o_low) memcpy(host + o_up, q->up, (size_t)n_items * 4);
+        if (has_w) {
+            memcpy(host + o_weighted, q->weighted, (size_t)Q);
+            memcpy(host + o_weight, q->weight, (size_t)n_items * 4);
+        }
+        memset(host + o_ctr, 0, kCtrWords * 4);
+        if ((e = cudaMemcpyAsync(dev, host, up_bytes, cudaMemcpyHostToDevice, s))) return cuda_fail(e, "query upload");
+        dq.item_off = (const int64_t *)(dev + o_item_off);
+        dq.out_off = (const int64_t *)(dev + o_out_off);
+        dq.k = q->k ? (const uint32_t *)(dev + o_k) : nullptr;
+        dq.dim = (const int32_t *)(dev + o_dim);
+        dq.low = (const int32_t *)(dev + o_low);
+        dq.up = (const int32_t *)(dev + o_up);
+        dq.weighted = has_w ? (const uint8_t *)(dev + o_weighted) : nullptr;
+        dq.weight = has_w ? (const float *)(dev + o_weight) : nullptr;
+    } else {
+#define H2D(dst, src, n) if ((n) > 0 && (e = cudaMemcpyAsync(dst, src, (size_t)(n), cudaMemcpyHostToDevice, s))) return cuda_fail(e, "query upload")
+        H2D(ws.item_off.p, q->item_off, (Q + 1) * 8);
+        H2D(ws.dim.p, q->dim, n_items * 4);
+        H2D(ws.low.p, q->low, n_items * 4);
+        H2D(ws.up.p, q->up, n_items * 4);
+        if (has_w) {
+            H2D(ws.weight.p, q->weight, n_items * 4);
+            H2D(ws.weighted.p, q->weighted, Q);
+        }
+        if (q->k) H2D(ws.k.p, q->k, Q * 4);
+        H2D(ws.out_off.p, out_off.data(), (Q + 1) * 8);
+#undef H2D
+        dq.item_off = (const int64_t *)ws.item_off.p;
+        dq.dim = (const int32_t *)ws.dim.p;
+        dq.low = (const int32_t *)ws.low.p;
+        dq.up = (const int32_t *)ws.up.p;
+        dq.weight = has_w ? (const float *)ws.weight.p : nullptr;
+        dq.weighted = has_w ? (const uint8_t *)ws.weighted.p : nullptr;
+        dq.k = q->k ? (const uint32_t *)ws.k.p : nullptr;
+        dq.out_off = (const int64_t *)ws.out_off.p;
+    }
     DeviceContext &ctx = device_context(ix->device);
     const DevIndex d = index_view(ix, ix->tuning);
     if (d.planes && (e = ws.reserve_planes(Q))) return cuda_fail(e, "search workspace");
     Work w = ws.view(Q, out_scores != nullptr);
-    ix->last_launches = launch_match(d, dq, w, ix->tuning, ctx.num_sms, s, nullptr, launch_need(ix, q));
+    if (small) {
+        w.ctr = (uint32_t *)(dev + o_ctr);
+        w.out_ids = (uint32_t *)(dev + o_ids);
+        w.out_counts = (uint32_t *)(dev + o_counts);
+        w.out_scores = out_scores ? (float *)(dev + o_scores) : nullptr;
+        w.out_cap = sumk;
+    }
+    ix->last_launches = launch_match(d, dq, w, ix->tuning, ctx.num_sms, s, nullptr,
+                                     launch_need(ix, q) | (small ? kCtrZeroed : 0u));
     if ((e = cudaGetLastError())) return cuda_fail(e, "match launch");
-    if ((e = cudaMemcpyAsync(ix->host_err, w.ctr + kCtrError, 4, cudaMemcpyDeviceToHost, s))) return cuda_fail(e, "error word");
-    if ((e = cudaMemcpyAsync(out_ids, w.out_ids, sumk * 4, cudaMemcpyDeviceToHost, s))) return cuda_fail(e, "result ids");
-    if ((e = cudaMemcpyAsync(out_counts, w.out_counts, sumk * 4, cudaMemcpyDeviceToHost, s))) return cuda_fail(e, "result counts");
-    if (out_scores && (e = cudaMemcpyAsync(out_scores, w.out_scores, sumk * 4, cudaMemcpyDeviceToHost, s)))
-        return cuda_fail(e, "result scores");
+    ix->call_results = -1;
+    if (small) {
+        if ((e = cudaMemcpyAsync(host + o_ctr, dev + o_ctr, at - o_ctr, cudaMemcpyDeviceToHost, s))) return cuda_fail(e, "results");
+        ix->call_results = sumk;
+        ix->call_ctr = o_ctr;
+    } else {
+        if ((e = cudaMemcpyAsync(ix->host_err, w.ctr + kCtrError, 4, cudaMemcpyDeviceToHost, s))) return cuda_fail(e, "error word");
+        if ((e = cudaMemcpyAsync(out_ids, w.out_ids, sumk * 4, cudaMemcpyDeviceToHost, s))) return cuda_fail(e, "result ids");
+        if ((e = cudaMemcpyAsync(out_counts, w.out_counts, sumk * 4, cudaMemcpyDeviceToHost, s))) return cuda_fail(e, "result counts");
+        if (out_scores && (e = cudaMemcpyAsync(out_scores, w.out_scores, sumk * 4, cudaMemcpyDeviceToHost, s)))
+            return cuda_fail(e, "result scores");
+    }
     if (!sync) return GENIE_OK;
     if ((e = cudaStreamSynchronize(s))) return cuda_fail(e, "search");
-    return check_device_error(*ix->host_err);
+    return finish_search(ix, out_ids, out_counts, out_scores);
 }
 
 }  // namespace gg
@@ -400,7 +478,7 @@ static genie_index *new_index() {
     genie_index *ix = new genie_index();
     ix->device = dev;
     ix->tuning = device_context(dev).tuning;
-    cudaMallocHost((void **)&ix->host_err, 16);
+    alloc_host_words(ix);
     return ix;
 }
 
@@ -615,7 +693,7 @@ int genie_search_multi(genie_index *const *ixs, const genie_queries *qs, int32_t
         if (qs[i].n_queries == 0 || custom[i]) continue;
         cudaError_t e = cudaStreamSynchronize(ixs[i]->stream);
         if (e && !rc) rc = cuda_fail(e, "multi-index search");
-        if (!rc) rc = check_device_error(*ixs[i]->host_err);
+        if (!rc) rc = finish_search(ixs[i], out_ids + base[i], out_counts + base[i], out_scores ? out_scores + base[i] : nullptr);
         ixs[i]->mu.unlock();
     }
     return rc;

@@ -42,15 +42,23 @@ struct Workspace {
     DevBuf out_ids, out_counts, out_scores;
     DevBuf counters;                 // per-object counters of a subsequence search
     DevBuf unit_key;
+    DevBuf call;                     // inputs, counters and results of a small call
     DevBuf planes;                   // per-query state of k_planes: bounds, histograms, key counts
     bool done_zeroed = false;
     int64_t done_q = 0;
-    cudaError_t reserve(int64_t Q, int64_t items, int64_t units, int64_t sumk);
+    // io: the query inputs and results too (a small call has its own, `call`)
+    cudaError_t reserve(int64_t Q, int64_t items, int64_t units, int64_t sumk, bool io = true);
     // what a search with an index's planes needs beside; before view()
     cudaError_t reserve_planes(int64_t Q);
     void release();
     Work view(int64_t Q, bool scores) const;
 };
+
+// Calls whose inputs and results fit are packed into one upload and one
+// download through pinned memory.
+constexpr size_t kCallBytes = 384 << 10;
+// The pinned words of an index (host_err).
+cudaError_t alloc_host_words(genie_index *ix);
 
 int validate_queries(const genie_queries *q, std::vector<int64_t> &out_off, int64_t &n_items);
 
@@ -121,7 +129,9 @@ struct genie_index {
     cudaStream_t stream = nullptr;
     std::mutex mu;                   // serialises searches on this handle's workspace
     gg::Workspace ws;
-    uint32_t *host_err = nullptr;    // pinned error word of the last search
+    uint32_t *host_err = nullptr;    // pinned: error word of the last search, then kCallBytes of a small call
+    int64_t call_results = -1;       // small call in flight: result slots (-1: none), and where its
+    size_t call_ctr = 0;             // counters and results start in the call's bytes
     int last_launches = 0;
     ~genie_index();
 };

@@ -143,7 +143,7 @@ int genie_index_create_compressed(const int32_t *values, int64_t n_objects, int3
     genie_index *ix = new genie_index();
     ix->device = dev;
     ix->tuning = device_context(dev).tuning;
-    cudaMallocHost((void **)&ix->host_err, 16);
+    alloc_host_words(ix);
     if (!build_host_index(values, n_objects, n_dims, ix->host)) {
         delete ix;
         return fail(GENIE_ERR_INVALID_ARG, "index build failed (N must be < 2^32)");

@@ -1554,8 +1554,8 @@ Tuning launch_tuning(const DevIndex &ix, const Tuning &tun, int num_sms) {
     return t;
 }
 
-int launch_plan(const DevIndex &ix, const DevQueries &Q, const Work &W, const Tuning &t, cudaStream_t s) {
-    cudaMemsetAsync(W.ctr, 0, kCtrWords * sizeof(uint32_t), s);
+int launch_plan(const DevIndex &ix, const DevQueries &Q, const Work &W, const Tuning &t, cudaStream_t s, bool zeroed) {
+    if (!zeroed) cudaMemsetAsync(W.ctr, 0, kCtrWords * sizeof(uint32_t), s);
     k_plan<<<Q.n_queries, kPlanThreads, 0, s>>>(ix, Q, W, t);
     return 1;
 }
@@ -1615,11 +1615,11 @@ int launch_kernel(int kern, const DevIndex &ix, const DevQueries &Q, const Work 
 int launch_match(const DevIndex &ix, const DevQueries &Q, const Work &W, const Tuning &tun,
                  int num_sms, cudaStream_t s, cudaEvent_t *ev, uint32_t need) {
     if (Q.n_queries <= 0) return 0;
-    if (!ix.planes || !W.lbk) need = kNeedLists;
+    if (!ix.planes || !W.lbk) need = kNeedLists | (need & kCtrZeroed);
     const Tuning t = launch_tuning(ix, tun, num_sms);
     int launches = 0;
     if (ev) cudaEventRecord(ev[0], s);
-    launches += launch_plan(ix, Q, W, t, s);
+    launches += launch_plan(ix, Q, W, t, s, (need & kCtrZeroed) != 0);
     if (ev) cudaEventRecord(ev[1], s);
     // dense last: sparse parts that overflow are re-queued to the dense lists
     for (int k = 0; k < kNumKern; ++k) {

@@ -25,7 +25,8 @@ constexpr int kStages = 4;
 // Whether the bitmap kernel's shared memory fits an id space of n objects.
 bool bitmap_fits(const Tuning &t, int64_t n_objects);
 // `need` may leave out kernels that would find no work on an index with planes.
-enum LaunchNeed : uint32_t { kNeedPlanes = 1, kNeedPlanesWeighted = 2, kNeedLists = 4, kNeedAll = 7 };
+// kCtrZeroed: the caller's upload has cleared W.ctr.
+enum LaunchNeed : uint32_t { kNeedPlanes = 1, kNeedPlanesWeighted = 2, kNeedLists = 4, kNeedAll = 7, kCtrZeroed = 8 };
 int launch_match(const DevIndex &ix, const DevQueries &Q, const Work &W, const Tuning &t,
                  int num_sms, cudaStream_t s, cudaEvent_t *ev = nullptr, uint32_t need = kNeedAll);
 

@@ -182,7 +182,7 @@ extern "C" int genie_index_load(const char *path, genie_index **out) {
     genie_index *ix = new genie_index();
     ix->device = dev;
     ix->tuning = device_context(dev).tuning;
-    cudaMallocHost((void **)&ix->host_err, 16);
+    alloc_host_words(ix);
     int rc = load_index(path, ix);
     if (rc) {
         delete ix;
