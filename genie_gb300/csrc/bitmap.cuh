@@ -419,7 +419,7 @@ __global__ void __launch_bounds__(kBmThreads, 1) k_bitmap(DevIndex ix, DevQuerie
             nres = n_hi;
         }
         if (failed) {
-            if (tid == 0) convert_to_dense(ix, W, T, q);
+            if (tid == 0) convert_to_dense(ix, Q, W, T, q);
         } else {
             for (uint32_t j = tid; j < k; j += kBmThreads) {
                 if (!GG_OK(out_off + j, W.out_cap, 4)) continue;

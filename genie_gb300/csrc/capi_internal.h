@@ -120,6 +120,7 @@ struct genie_index {
     gg::DevBuf d_dir_slot, d_dir_row_key;
     bool bm_ready = false;
     int64_t bm_words = 0;
+    uint32_t bm_zero = 0;
     gg::DevBuf d_bm_slot, d_bm_rows;
     std::vector<std::pair<int32_t, gg::DevBuf *>> dirs;
     int64_t pl_bytes = -1;           // what the planes take (0: the index has none, -1: not looked at)

@@ -83,12 +83,15 @@ struct DevIndex {
     const uint32_t *dir32;
     int32_t dir8_tile;
     int32_t dir32_tile;
-    // presence bitmaps of the dense lists (tile_dir.cu): bm_slot[key] = row of
-    // a list holding >= 1/16 of the objects (~0u: none); a row is bm_words
-    // words, bit o set when object o is listed.  Null when absent.
+    // presence bitmaps of the dense lists (tile_dir.cu): bm_slot[key] = first
+    // row of the list (low 28 bits) and its rows less one (high four), ~0u for
+    // a list without; a row is bm_words words (a multiple of four), bit o of
+    // its row r set when object o is listed more than r times.  Row bm_zero is
+    // empty.  Null when absent.
     const uint32_t *bm_slot;
     const uint32_t *bm_rows;
     int64_t bm_words;
+    uint32_t bm_zero;
     // cumulative presence planes of a byte-valued index (planes.cu): in every
     // tile of kPlTile objects, one row of pl_row_vec 16-byte vectors per key,
     // then an empty and a full row.  Null when absent.

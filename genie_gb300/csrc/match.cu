@@ -43,14 +43,25 @@ constexpr int kPlanThreads = 256;
 
 // Id-range parts of a dense query: each sweeps T.dense_part_work objects in
 // whole counter tiles (at least one), at most W.max_parts parts.  Fewer,
-// longer parts pay a part's setup and merge less often and let its later
-// tiles merge against a full running top-k.  Every dense query of one
-// counter width has the same number, so that the dense kernel can take its
-// work part-major (take_dense).
-__device__ __forceinline__ int64_t dense_parts(const DevIndex &ix, const Work &W, const Tuning &T, bool small) {
+// longer parts pay a part's setup and merge less often (16,000 cycles of a
+// part of one tile) and let its later tiles merge against a full running
+// top-k, so a batch of nq queries takes as long ones as leave four parts a
+// CTA, and parts whose share of the index (4 bytes an id, about one
+// compressed) stays within kPartSlice, which L2 keeps while the batch counts
+// them (short texts, 1,000,000 x 32, 1,024 queries: 1.38 ms with a tile a
+// part, 1.03 with the query whole).  Every dense query of one counter width
+// has the same number, so that the dense kernel can take its work part-major
+// (take_dense).
+constexpr int64_t kPartSlice = 48 << 20;
+__device__ __forceinline__ int64_t dense_parts(const DevIndex &ix, const DevQueries &Q, const Work &W, const Tuning &T,
+                                               bool small) {
     const int64_t tile = small ? T.dense_tile_u8 : T.dense_tile_u32;
     const int64_t ntiles = (ix.n_objects + tile - 1) / tile;
-    int64_t per = T.dense_part_work / tile;
+    const int64_t nq = Q.dyn ? (int64_t)Q.dyn[0] : (int64_t)Q.n_queries;
+    const int64_t fill = (4 * (int64_t)T.num_sms + nq - 1) / (nq > 0 ? nq : 1);
+    const int64_t slices = (ix.n_ids * (ix.codec ? 1 : 4) + kPartSlice - 1) / kPartSlice;
+    int64_t per = ntiles / (fill > slices ? fill : slices);
+    if (per < T.dense_part_work / tile) per = T.dense_part_work / tile;
     if (per < 1) per = 1;
     const int64_t np = (ntiles + per - 1) / per;
     const int64_t pd = np < W.max_parts ? np : W.max_parts;
@@ -333,7 +344,7 @@ __global__ void __launch_bounds__(kPlanThreads, 8) k_plan(DevIndex ix, DevQuerie
                 list = packed ? kListSparsePacked : kListSparseWide;
             } else {
                 qi.cls = kClsDense;
-                qi.parts = (uint16_t)dense_parts(ix, W, T, small);
+                qi.parts = (uint16_t)dense_parts(ix, Q, W, T, small);
                 list = small ? kListDenseSmall : kListDenseWide;
             }
         }
@@ -820,10 +831,10 @@ struct MergeSet {
     }
 };
 
-__device__ void convert_to_dense(const DevIndex &ix, const Work &W, const Tuning &T, uint32_t q) {
+__device__ void convert_to_dense(const DevIndex &ix, const DevQueries &Q, const Work &W, const Tuning &T, uint32_t q) {
     QInfo qi = W.qinfo[q];
     const bool small = (qi.flags & kFlagSmallCount) != 0;
-    qi.parts = (uint16_t)dense_parts(ix, W, T, small);
+    qi.parts = (uint16_t)dense_parts(ix, Q, W, T, small);
     qi.cls = kClsDense;
     W.qinfo[q] = qi;
     W.done[q] = 0;
@@ -864,7 +875,7 @@ __device__ void finish_part(const DevIndex &ix, const Work &W, const Tuning &T, 
     if (!ss.sc[12]) return;
     __threadfence();
     if (atomicAdd(&W.qstate[q], 0u) & 1u) {       // a sparse part overflowed: redo densely
-        if (threadIdx.x == 0) convert_to_dense(ix, W, T, q);
+        if (threadIdx.x == 0) convert_to_dense(ix, Q, W, T, q);
         __syncthreads();
         return;
     }
@@ -1114,6 +1125,149 @@ struct TileSet {
     }
 };
 
+// Byte counters of a tile's bitmap rows: vector v of 128 objects a thread, so
+// the adds need no atomics.  The rows' bits are summed bit-sliced (plane t
+// holds bit t of each object's count so far, at most 31 rows a pass) by a
+// carry-save adder tree, four rows of 16-byte loads in flight; each nibble of
+// the planes is then spread into its four counter bytes, which are stored
+// (first pass over a tile's counters, which then need no clearing) or added
+// to, 16 at a time.  A word a thread, eight rows in flight and byte-word adds
+// on a cleared tile took 25,000 cycles a tile of 147,456 objects (14 rows,
+// five dependent rounds of loads, eight-way bank conflicts); this takes 18,000.
+__device__ __forceinline__ void bitmap_counts(const uint32_t *__restrict__ rows, int64_t words, const uint32_t *bm_row,
+                                              uint32_t nbm, uint32_t nvec, bool fresh, uint4 *c4) {
+    constexpr int R = 4;      // rows the adder tree takes at once
+    auto csa = [](uint32_t &s, uint32_t &c, uint32_t a, uint32_t b, uint32_t d) {
+        c = (a & b) | (a & d) | (b & d);
+        s = a ^ b ^ d;
+    };
+    // The planes of 32 objects as 32 counter bytes: an 8 x 8 bit transpose in
+    // each byte column (planes 5 to 7 are empty), then the bytes into order.
+    // Spreading nibbles by multiplication took three times the instructions.
+    auto flush = [&](uint32_t p0, uint32_t p1, uint32_t p2, uint32_t p3, uint32_t p4, uint4 *dst, bool store) {
+        uint32_t a[8] = {p0, p1, p2, p3, p4, 0, 0, 0};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const uint32_t t = ((a[i] >> 4) ^ a[i + 4]) & 0x0F0F0F0Fu;
+            a[i + 4] ^= t;
+            a[i] ^= t << 4;
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int i = (k & 1) | (k & 2) << 1;
+            const uint32_t t = ((a[i] >> 2) ^ a[i + 2]) & 0x33333333u;
+            a[i + 2] ^= t;
+            a[i] ^= t << 2;
+        }
+#pragma unroll
+        for (int i = 0; i < 8; i += 2) {
+            const uint32_t t = ((a[i] >> 1) ^ a[i + 1]) & 0x55555555u;
+            a[i + 1] ^= t;
+            a[i] ^= t << 1;
+        }
+        // byte c of a[r] counts object 8 c + r
+        uint32_t out[8];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const uint32_t x = __byte_perm(a[4 * h], a[4 * h + 1], 0x5140), y = __byte_perm(a[4 * h], a[4 * h + 1], 0x7362);
+            const uint32_t z = __byte_perm(a[4 * h + 2], a[4 * h + 3], 0x5140);
+            const uint32_t w = __byte_perm(a[4 * h + 2], a[4 * h + 3], 0x7362);
+            out[h] = __byte_perm(x, z, 0x5410);
+            out[2 + h] = __byte_perm(x, z, 0x7632);
+            out[4 + h] = __byte_perm(y, w, 0x5410);
+            out[6 + h] = __byte_perm(y, w, 0x7632);
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            uint4 v = store ? make_uint4(0, 0, 0, 0) : dst[h];
+            v.x += out[4 * h];
+            v.y += out[4 * h + 1];
+            v.z += out[4 * h + 2];
+            v.w += out[4 * h + 3];
+            dst[h] = v;
+        }
+    };
+    // the vectors past the last whole round of the block go a word a thread, so
+    // that they too keep most threads busy (eight rows of loads in flight)
+    const uint32_t whole = nvec >= blockDim.x ? nvec / blockDim.x * blockDim.x : 0u;
+    for (uint32_t j = 4 * whole + threadIdx.x; j < 4 * nvec; j += blockDim.x) {
+        uint32_t p[5] = {0, 0, 0, 0, 0}, in_pass = 0;
+        bool store = fresh;
+        for (uint32_t u0 = 0; u0 < nbm; u0 += 8) {
+            uint32_t x[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) x[i] = u0 + i < nbm ? __ldg(rows + (size_t)bm_row[u0 + i] * (size_t)words + j) : 0u;
+#pragma unroll
+            for (int i = 0; i < 8; i += 4) {
+                uint32_t a, b, c;
+                csa(p[0], a, p[0], x[i], x[i + 1]);
+                csa(p[0], b, p[0], x[i + 2], x[i + 3]);
+                csa(p[1], c, p[1], a, b);
+#pragma unroll
+                for (int t = 2; t < 5; ++t) {
+                    const uint32_t y = p[t];
+                    p[t] = y ^ c;
+                    c &= y;
+                }
+            }
+            in_pass += 8;
+            if (in_pass + 8 > 31 || u0 + 8 >= nbm) {
+                flush(p[0], p[1], p[2], p[3], p[4], c4 + 2 * j, store);
+                p[0] = p[1] = p[2] = p[3] = p[4] = 0;
+                store = false;
+                in_pass = 0;
+            }
+        }
+    }
+    for (uint32_t v = threadIdx.x; v < whole; v += blockDim.x) {
+        uint32_t p[5][4];
+#pragma unroll
+        for (int t = 0; t < 5; ++t)
+#pragma unroll
+            for (int w = 0; w < 4; ++w) p[t][w] = 0;
+        bool store = fresh;
+        uint32_t in_pass = 0;
+        auto load = [&](uint32_t u) {
+            return u < nbm ? __ldg((const uint4 *)(rows + (size_t)bm_row[u] * (size_t)words) + v) : make_uint4(0, 0, 0, 0);
+        };
+        uint4 n[R];            // the next four rows load while these are summed
+#pragma unroll
+        for (int i = 0; i < R; ++i) n[i] = load(i);
+        for (uint32_t u0 = 0; u0 < nbm; u0 += R) {
+            uint4 x[R];
+#pragma unroll
+            for (int i = 0; i < R; ++i) x[i] = n[i];
+#pragma unroll
+            for (int i = 0; i < R; ++i) n[i] = load(u0 + R + i);
+#pragma unroll
+            for (int w = 0; w < 4; ++w) {
+                uint32_t a, b, c;
+                csa(p[0][w], a, p[0][w], (&x[0].x)[w], (&x[1].x)[w]);
+                csa(p[0][w], b, p[0][w], (&x[2].x)[w], (&x[3].x)[w]);
+                csa(p[1][w], c, p[1][w], a, b);
+#pragma unroll
+                for (int t = 2; t < 5; ++t) {
+                    const uint32_t y = p[t][w];
+                    p[t][w] = y ^ c;
+                    c &= y;
+                }
+            }
+            in_pass += R;
+            if (in_pass + R > 31 || u0 + R >= nbm) {
+#pragma unroll
+                for (int w = 0; w < 4; ++w)
+                    flush(p[0][w], p[1][w], p[2][w], p[3][w], p[4][w], c4 + 8 * v + 2 * w, store);
+#pragma unroll
+                for (int t = 0; t < 5; ++t)
+#pragma unroll
+                    for (int w = 0; w < 4; ++w) p[t][w] = 0;
+                store = false;
+                in_pass = 0;
+            }
+        }
+    }
+}
+
 // Id-tiled dense counters in shared memory; one CTA sweeps the tiles of one
 // query part, keeping its running top-k.  Replaces the per-query global bitmap
 // (match.cu:276-294, match_device_utils.h:422-446), which wraps above
@@ -1140,16 +1294,18 @@ __device__ __forceinline__ void dense_list(const DevIndex &ix, const DevQueries 
     uint32_t *bm_row = (uint32_t *)(it_raw + kItemChunk * 28 + 16 + sizeof(SelectScratch));
     uint32_t *bm_inc = bm_row + kItemChunk;
     uint32_t *unit_bm = bm_inc + kItemChunk;
-    __shared__ uint32_t s_q, s_p, s_nS, s_nc, s_L, s_nbm;
+    // and where its list starts
+    int64_t *unit_s0 = (int64_t *)(unit_bm + kItemChunk);
+    __shared__ uint32_t s_q, s_p, s_nS, s_nc, s_L, s_nbm, s_fit;
 
     const int list = SMALL ? kListDenseSmall : kListDenseWide;
-    const uint32_t P_list = (uint32_t)dense_parts(ix, W, T, SMALL);
+    const uint32_t P_list = (uint32_t)dense_parts(ix, Q, W, T, SMALL);
     // the tile directory of this counter width, when built for this tile size
     const uint32_t *dir = SMALL ? ix.dir8 : ix.dir32;
     const bool use_dir = dir != nullptr && ix.dir_slot != nullptr && W.unit_key != nullptr &&
                          (SMALL ? ix.dir8_tile : ix.dir32_tile) == (int32_t)tile_cap;
     // dense lists counted from their bitmaps (tiles start at a word boundary)
-    const bool use_bm = ix.bm_slot != nullptr && W.unit_key != nullptr && tile_cap % 32u == 0 &&
+    const bool use_bm = ix.bm_slot != nullptr && W.unit_key != nullptr && tile_cap % 128u == 0 &&
                         (T.dense_bitmaps & (SMALL ? 1 : 2)) != 0;
     for (;;) {
         if (tid == 0) {
@@ -1157,6 +1313,7 @@ __device__ __forceinline__ void dense_list(const DevIndex &ix, const DevQueries 
             if (!take_dense(W, list, P_list, wk)) wk.x = 0xFFFFFFFFu;
             s_q = wk.x;
             s_p = wk.y;
+            s_fit = 0;
         }
         __syncthreads();
         const uint32_t q = s_q, p = s_p;
@@ -1179,7 +1336,14 @@ __device__ __forceinline__ void dense_list(const DevIndex &ix, const DevQueries 
         if (single && (int32_t)tid < qi.n_units) {
             const int64_t it = qi.unit0 + tid;
             const int64_t s0 = W.span_start[it], e0 = s0 + W.span_len[it];
-            unit_bm[tid] = (use_bm && e0 > s0) ? ix.bm_slot[W.unit_key[it]] : 0xFFFFFFFFu;
+            unit_s0[tid] = s0;
+            st.inc[tid] = W.inc[it];
+            uint32_t bm = (use_bm && e0 > s0) ? ix.bm_slot[W.unit_key[it]] : 0xFFFFFFFFu;
+            // more rows than a chunk holds: the rest of the lists keep to their
+            // ids, in every tile alike (their cursors move on tile by tile)
+            if (bm != 0xFFFFFFFFu && atomicAdd(&s_fit, (bm >> 28) + 1u) + (bm >> 28) + 1u > (uint32_t)kItemChunk)
+                bm = 0xFFFFFFFFu;
+            unit_bm[tid] = bm;
             const uint32_t row = (use_dir && e0 > s0) ? ix.dir_slot[W.unit_key[it]] : 0xFFFFFFFFu;
             cur[tid] = row != 0xFFFFFFFFu ? -1 - (int64_t)row
                                           : ((t0 == 0 || e0 == s0) ? s0
@@ -1195,30 +1359,39 @@ __device__ __forceinline__ void dense_list(const DevIndex &ix, const DevQueries 
             const uint32_t tile_hi = (uint32_t)umin64(N, (t + 1) * tile_cap);
             const uint32_t n_ids = tile_hi - tile_lo;
             const uint32_t n_pad = (n_ids + 15) & ~15u;
-            // zero the counters of this tile
             uint4 *c4 = (uint4 *)cnt;
             const uint32_t n4 = (n_pad * (SMALL ? 1 : 4)) / 16;
-            for (uint32_t i = tid; i < n4; i += blockDim.x) c4[i] = make_uint4(0, 0, 0, 0);
             bool any_ids = false;
             for (int32_t c0 = 0; c0 < qi.n_units; c0 += kItemChunk) {
                 const int32_t mc = min(kItemChunk, qi.n_units - c0);
                 uint32_t len = 0;
                 if ((int32_t)tid < mc) {
                     const int64_t it = qi.unit0 + c0 + tid;
-                    const int64_t s0 = W.span_start[it], e0 = s0 + W.span_len[it];
+                    const int64_t s0 = single ? unit_s0[tid] : W.span_start[it];
+                    auto e0 = [&] { return s0 + W.span_len[it]; };
+                    const uint32_t inc = single ? st.inc[tid] : W.inc[it];
                     uint32_t row = 0xFFFFFFFFu;
                     if (single) {
                         if (cur[tid] < 0) row = (uint32_t)(-1 - cur[tid]);
-                    } else if (use_dir && e0 > s0) {
+                    } else if (use_dir && e0() > s0) {
                         row = ix.dir_slot[W.unit_key[it]];
                     }
                     int64_t a, b;
                     const uint32_t brow = single ? unit_bm[tid]
-                                                 : ((use_bm && e0 > s0) ? ix.bm_slot[W.unit_key[it]] : 0xFFFFFFFFu);
-                    if (brow != 0xFFFFFFFFu) {          // counted from its bitmap, not streamed
-                        const uint32_t at = atomicAdd(&s_nbm, 1u);
-                        bm_row[at] = brow;
-                        bm_inc[at] = W.inc[it];
+                                                 : ((use_bm && e0() > s0) ? ix.bm_slot[W.unit_key[it]] : 0xFFFFFFFFu);
+                    // counted from its bitmaps, not streamed (unless they are
+                    // more than the chunk holds)
+                    bool mapped = false;
+                    if (brow != 0xFFFFFFFFu) {
+                        const uint32_t first = brow & 0x0FFFFFFFu, rows = (brow >> 28) + 1u;
+                        const uint32_t at = atomicAdd(&s_nbm, rows);
+                        mapped = at + rows <= (uint32_t)kItemChunk;
+                        for (uint32_t r = 0; r < rows && at + r < (uint32_t)kItemChunk; ++r) {
+                            bm_row[at + r] = mapped ? first + r : ix.bm_zero;
+                            bm_inc[at + r] = inc;
+                        }
+                    }
+                    if (mapped) {
                         a = b = s0;
                     } else if (row != 0xFFFFFFFFu) {
                         // the tile's cut from the directory: the first id (segment) at or past
@@ -1228,13 +1401,13 @@ __device__ __forceinline__ void dense_list(const DevIndex &ix, const DevQueries 
                         a = s0 + (ix.codec ? (fa ? fa - 1 : 0) : fa);
                         b = s0 + fb;
                     } else {
-                        a = single ? cur[tid] : (t == 0 ? s0 : first_unit(ix, s0, e0, tile_lo));
-                        b = (tile_hi >= N) ? e0 : next_unit_near(ix, a, s0, e0, tile_lo, tile_hi, N);
+                        a = single ? cur[tid] : (t == 0 ? s0 : first_unit(ix, s0, e0(), tile_lo));
+                        b = (tile_hi >= N) ? e0() : next_unit_near(ix, a, s0, e0(), tile_lo, tile_hi, N);
                         // a compressed segment may straddle tile_hi: the next tile starts at it again
                         if (single) cur[tid] = (ix.codec && b > a) ? b - 1 : b;
                     }
                     st.start[tid] = a;
-                    st.inc[tid] = W.inc[it];
+                    st.inc[tid] = inc;
                     len = (uint32_t)(b - a);
                     st.len[tid] = len;
                 }
@@ -1246,81 +1419,32 @@ __device__ __forceinline__ void dense_list(const DevIndex &ix, const DevQueries 
                 if (tid == 0) st.flat[mc] = tot;
                 __syncthreads();
                 if (tot) any_ids = true;
-                // dense lists from their bitmaps: thread j owns the tile's objects
-                // 32j .. 32j+31 (counter words 8j .. 8j+7, or 32j .. 32j+31), so the
-                // adds need no atomics; the id stream below waits for them
-                const uint32_t nbm = s_nbm;
+                // dense lists from their bitmaps; the id stream below waits for them
+                const uint32_t nbm = min(s_nbm, (uint32_t)kItemChunk);
+                // byte counters: the first chunk's bitmaps store every counter of the tile
+                const bool fresh = SMALL && nbm && c0 == 0;
+                if (c0 == 0 && !fresh) {
+                    for (uint32_t i = tid; i < n4; i += blockDim.x) c4[i] = make_uint4(0, 0, 0, 0);
+                    __syncthreads();
+                }
                 if (nbm) {
                     any_ids = true;
                     const uint32_t *rows = ix.bm_rows + (tile_lo >> 5);
-                    const uint32_t nwords = (n_ids + 31) >> 5;
-                    constexpr uint32_t kBmLoads = 8;      // bitmap words in flight per thread
-                    static_assert(kBmLoads == 8, "the adder tree takes eight rows a group");
-                    for (uint32_t j = tid; j < nwords; j += blockDim.x) {
-                        // byte counters: the lists' bits are summed bit-sliced (plane t holds
-                        // bit t of each object's count so far, at most 24 lists a pass), then
-                        // each nibble of the planes is spread into its four counter bytes
-                        uint32_t p0 = 0, p1 = 0, p2 = 0, p3 = 0, p4 = 0, in_pass = 0;
-                        // the next group's words load while this group is summed
-                        uint32_t wn[kBmLoads];
-#pragma unroll
-                        for (uint32_t i = 0; i < kBmLoads; ++i)
-                            wn[i] = i < nbm ? __ldg(rows + (size_t)bm_row[i] * (size_t)ix.bm_words + j) : 0u;
-                        for (uint32_t u0 = 0; u0 < nbm; u0 += kBmLoads) {
-                            uint32_t w[kBmLoads];
-#pragma unroll
-                            for (uint32_t i = 0; i < kBmLoads; ++i) w[i] = wn[i];
-#pragma unroll
-                            for (uint32_t i = 0; i < kBmLoads; ++i)
-                                wn[i] = u0 + kBmLoads + i < nbm
-                                            ? __ldg(rows + (size_t)bm_row[u0 + kBmLoads + i] * (size_t)ix.bm_words + j)
-                                            : 0u;
-                            if (SMALL) {
-                                // the eight rows' bits into the planes by a carry-save adder
-                                // tree (full adders: sum a^b^c, carry majority(a,b,c)); a group
-                                // adds at most 8, so one weight-8 carry ripples into p3, p4
-                                auto csa = [](uint32_t &s, uint32_t &c, uint32_t a, uint32_t b, uint32_t d) {
-                                    const uint32_t u = a ^ b;
-                                    s = u ^ d;
-                                    c = (a & b) | (u & d);
-                                };
-                                uint32_t t2a, t2b, t2c, t2d, t4a, t4b, t8;
-                                csa(p0, t2a, p0, w[0], w[1]);
-                                csa(p0, t2b, p0, w[2], w[3]);
-                                csa(p1, t4a, p1, t2a, t2b);
-                                csa(p0, t2c, p0, w[4], w[5]);
-                                csa(p0, t2d, p0, w[6], w[7]);
-                                csa(p1, t4b, p1, t2c, t2d);
-                                csa(p2, t8, p2, t4a, t4b);
-                                const uint32_t c3 = p3 & t8;
-                                p3 ^= t8;
-                                p4 ^= c3;
-                                in_pass += kBmLoads;
-                                if (in_pass + kBmLoads > 31 || u0 + kBmLoads >= nbm) {
-#pragma unroll
-                                    for (int k = 0; k < 8; ++k) {
-                                        auto spread = [](uint32_t x) { return (x * 0x00204081u) & 0x01010101u; };
-                                        const int sh = 4 * k;
-                                        cnt[8 * j + k] += spread((p0 >> sh) & 15u) + (spread((p1 >> sh) & 15u) << 1) +
-                                                          (spread((p2 >> sh) & 15u) << 2) + (spread((p3 >> sh) & 15u) << 3) +
-                                                          (spread((p4 >> sh) & 15u) << 4);
-                                    }
-                                    p0 = p1 = p2 = p3 = p4 = 0;
-                                    in_pass = 0;
-                                }
-                            } else {
-#pragma unroll
-                                for (uint32_t i = 0; i < kBmLoads; ++i) {
-                                    const uint32_t inc = u0 + i < nbm ? bm_inc[u0 + i] : 0u;
-                                    uint32_t x = w[i];
-                                    while (x) {
-                                        const uint32_t bit = (uint32_t)__ffs((int)x) - 1u;
-                                        cnt[32 * j + bit] += inc;
-                                        x &= x - 1u;
-                                    }
+                    if (SMALL) {
+                        bitmap_counts(rows, ix.bm_words, bm_row, nbm, (n_ids + 127) >> 7, fresh, c4);
+                    } else {
+                        // four-byte counters: a word of 32 objects a thread
+                        const uint32_t nwords = (n_ids + 31) >> 5;
+                        for (uint32_t j = tid; j < nwords; j += blockDim.x)
+                            for (uint32_t u = 0; u < nbm; ++u) {
+                                const uint32_t inc = bm_inc[u];
+                                uint32_t x = __ldg(rows + (size_t)bm_row[u] * (size_t)ix.bm_words + j);
+                                while (x) {
+                                    const uint32_t bit = (uint32_t)__ffs((int)x) - 1u;
+                                    cnt[32 * j + bit] += inc;
+                                    x &= x - 1u;
                                 }
                             }
-                        }
                     }
                     __syncthreads();
                     if (tid == 0) s_nbm = 0;
@@ -1469,7 +1593,7 @@ size_t sparse_smem_bytes(const Tuning &t, bool packed) {
 size_t dense_smem_bytes(const Tuning &t, bool small) {
     size_t c = (size_t)(small ? t.dense_tile_u8 : t.dense_tile_u32 * 4);
     return c + (size_t)kMaxK * 8 + (size_t)kCandCap * 8 + kItemChunk * 28 + 16 + sizeof(SelectScratch) + kItemChunk * 12 +
-           64;
+           kItemChunk * 8 + 64;
 }
 
 Tuning default_tuning() {

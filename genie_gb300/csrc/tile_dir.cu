@@ -18,15 +18,19 @@
 // thread per (row, boundary) and kept while the index lives: batches capture
 // its address in their CUDA graphs.
 //
-// Dense-list bitmaps: a posting list holding at least 1/16 of the objects
-// (the lists of a dimension's most common value) is also kept as a presence
-// bitmap of n_objects bits, a tenth or less of its ids' bytes at such
-// densities.  The dense kernel counts such a list from its bitmap words
-// (each thread owns 32 objects of the tile, so plain adds replace the
-// shared-memory atomics) and streams (or decodes) only the other lists.
-// Built once per index with one value per object and dim (no list repeats an
-// id; a compressed index decodes its dense lists' segments to build them), on
-// first use, within a budget; kept while the index lives.
+// Dense-list bitmaps: a posting list holding at least 1/64 (compressed 1/128) of the
+// objects (the lists of a dimension's common values) is also kept as a
+// presence bitmap of n_objects bits.  The dense kernel counts such a list from
+// its bitmap words (each thread owns a vector of objects of the tile, so plain
+// adds replace the shared-memory atomics) and streams (or decodes) only the
+// other lists.  A word of 32 objects costs about four instructions however
+// many of them are listed, a decoded id one or two and an atomic, hence the
+// density: short texts in 1,000,000 x 32, 1,024 queries, 1.70 ms in the dense
+// kernel with lists of 1/16 and more, 1.47 with 1/64, 1.45 with 1/128 and
+// 1/256.  A bag index may list an object more than once: row r of a list marks
+// the objects listed more than r times, so the rows add up to the counts.
+// Built once per index (a compressed index decodes its dense lists' segments),
+// on first use, within a budget; kept while the index lives.
 #include "capi_internal.h"
 #include "codecs.cuh"
 
@@ -45,19 +49,42 @@ constexpr int64_t kDirMinLens[] = {1, 16, 64, 256, 1024, 4096};
 // smallest autotuner tile)
 constexpr int64_t kDirSmallestTile = 98304 / 4;
 constexpr int64_t kBmMinObjects = 65536;         // id spaces too small for bitmaps to pay
-constexpr int64_t kBmDensity = 16;               // a list with len * 16 >= n_objects gets a bitmap
+// A list with len * density >= n_objects (* rows) gets bitmaps; on a table that
+// will have planes only the densest do (its lists are counted until then).
+constexpr int64_t kBmDensityPlain = 64, kBmDensityCompressed = 128, kBmDensityPlanes = 16;
+constexpr uint32_t kBmMaxRows = 16;              // most rows of a list (an object listed more often: none)
 constexpr size_t kBmBudget = size_t(2) << 30;    // bytes of all bitmap rows at most
 
-// Bit o of row r for every id o of row r's list; one CTA row per blockIdx.y.
-__global__ void k_bm_build(const uint32_t *__restrict__ ids, const int64_t *__restrict__ key_off,
-                           const uint32_t *__restrict__ row_key, int64_t words, uint32_t *__restrict__ rows) {
-    const uint32_t r = blockIdx.y;
-    const uint32_t key = row_key[r];
+// Most times one id repeats in each listed list (ids sorted, so the repeats
+// are neighbours); one list per blockIdx.y.
+__global__ void k_bm_levels(const uint32_t *__restrict__ ids, const int64_t *__restrict__ key_off,
+                            const uint32_t *__restrict__ row_key, uint32_t *__restrict__ most) {
+    const uint32_t key = row_key[blockIdx.y];
     const int64_t a = key_off[key], e = key_off[key + 1];
-    uint32_t *row = rows + (size_t)r * (size_t)words;
+    uint32_t top = 0;
     for (int64_t p = a + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < e; p += (int64_t)gridDim.x * blockDim.x) {
         const uint32_t id = ids[p];
-        atomicOr(&row[id >> 5], 1u << (id & 31u));
+        uint32_t run = 1;
+        while (run <= kBmMaxRows && p - (int64_t)run >= a && ids[p - run] == id) ++run;
+        top = max(top, run);
+    }
+    top = __reduce_max_sync(0xffffffffu, top);
+    if ((threadIdx.x & 31) == 0) atomicMax(&most[blockIdx.y], top);
+}
+
+// Bit o of row r for the r-th listing of every id o in a list (at most `limit`
+// rows before it are looked at); one list per blockIdx.y, its first row given.
+__global__ void k_bm_build(const uint32_t *__restrict__ ids, const int64_t *__restrict__ key_off,
+                           const uint32_t *__restrict__ row_key, const uint32_t *__restrict__ first, uint32_t limit,
+                           int64_t words, uint32_t *__restrict__ rows) {
+    const uint32_t key = row_key[blockIdx.y];
+    const int64_t a = key_off[key], e = key_off[key + 1];
+    uint32_t *row = rows + (size_t)first[blockIdx.y] * (size_t)words;
+    for (int64_t p = a + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < e; p += (int64_t)gridDim.x * blockDim.x) {
+        const uint32_t id = ids[p];
+        uint32_t r = 0;
+        while (r + 1 < limit && p - (int64_t)r - 1 >= a && ids[p - r - 1] == id) ++r;
+        atomicOr(&row[(size_t)r * (size_t)words + (id >> 5)], 1u << (id & 31u));
     }
 }
 
@@ -176,48 +203,71 @@ bool dense_bitmaps(genie_index *ix) {
     ix->bm_ready = true;
     ix->bm_words = 0;
     const int64_t n = ix->host.n_objects, nk = ix->host.n_keys();
-    if (ix->is_bag || ix->sub_shift >= 0 || n < kBmMinObjects || nk <= 0 ||
-        nk >= (int64_t)0xFFFFFFFFll)
-        return false;
-    const int64_t words = (n + 31) / 32;
-    std::vector<uint32_t> slot((size_t)nk, 0xFFFFFFFFu), row_key;
-    for (int64_t k = 0; k < nk; ++k)
-        if ((ix->host.key_off[k + 1] - ix->host.key_off[k]) * kBmDensity >= n &&
-            (row_key.size() + 1) * (size_t)words * 4 <= kBmBudget && row_key.size() < 65535) {
-            slot[(size_t)k] = (uint32_t)row_key.size();
-            row_key.push_back((uint32_t)k);
-        }
-    if (row_key.empty()) return false;
-    DevBuf rk;
-    cudaError_t e;
-    if ((e = ix->d_bm_slot.reserve(slot.size() * 4)) ||
-        (e = cudaMemcpy(ix->d_bm_slot.p, slot.data(), slot.size() * 4, cudaMemcpyHostToDevice)) ||
-        (e = rk.reserve(row_key.size() * 4)) ||
-        (e = cudaMemcpy(rk.p, row_key.data(), row_key.size() * 4, cudaMemcpyHostToDevice)) ||
-        (e = ix->d_bm_rows.reserve(row_key.size() * (size_t)words * 4)) ||
-        (e = cudaMemsetAsync(ix->d_bm_rows.p, 0, row_key.size() * (size_t)words * 4, ix->stream))) {
+    if (ix->sub_shift >= 0 || n < kBmMinObjects || nk <= 0 || nk >= (int64_t)0xFFFFFFFFll) return false;
+    const int64_t words = (n + 127) / 128 * 4;
+    const int64_t density = ix->pl_bytes > 0 ? kBmDensityPlanes : ix->codec ? kBmDensityCompressed : kBmDensityPlain;
+    // the dense lists, and the rows each needs
+    std::vector<uint32_t> key;
+    for (int64_t k = 0; k < nk && key.size() < 65535; ++k)
+        if ((ix->host.key_off[k + 1] - ix->host.key_off[k]) * density >= n) key.push_back((uint32_t)k);
+    if (key.empty()) return false;
+    std::vector<uint32_t> most(key.size(), 1u);
+    const unsigned lists = (unsigned)key.size();
+    DevBuf rk, mr;
+    cudaError_t e = cudaSuccess;
+    auto give_up = [&] {
         cudaGetLastError();
         rk.release();
+        mr.release();
         ix->d_bm_slot.release();
         ix->d_bm_rows.release();
         return false;
+    };
+    if ((e = rk.reserve(lists * 4)) || (e = mr.reserve(lists * 4)) ||
+        (e = cudaMemcpy(rk.p, key.data(), lists * 4, cudaMemcpyHostToDevice)))
+        return give_up();
+    if (ix->is_bag) {
+        if ((e = cudaMemsetAsync(mr.p, 0, lists * 4, ix->stream))) return give_up();
+        k_bm_levels<<<dim3(64, lists), 256, 0, ix->stream>>>(ix->dev.ids, ix->dev.key_off, (const uint32_t *)rk.p,
+                                                             (uint32_t *)mr.p);
+        if (cudaGetLastError() || cudaStreamSynchronize(ix->stream) ||
+            cudaMemcpy(most.data(), mr.p, lists * 4, cudaMemcpyDeviceToHost))
+            return give_up();
     }
-    if (ix->codec)
+    std::vector<uint32_t> slot((size_t)nk, 0xFFFFFFFFu), row_key, first;
+    uint32_t n_rows = 0;
+    for (uint32_t i = 0; i < lists; ++i) {
+        const int64_t len = ix->host.key_off[key[i] + 1] - ix->host.key_off[key[i]];
+        if (most[i] > kBmMaxRows || len * density < n * (int64_t)most[i] ||
+            ((size_t)n_rows + most[i] + 1) * (size_t)words * 4 > kBmBudget)
+            continue;
+        slot[key[i]] = n_rows | (most[i] - 1) << 28;
+        row_key.push_back(key[i]);
+        first.push_back(n_rows);
+        n_rows += most[i];
+    }
+    if (row_key.empty()) return give_up();
+    const size_t row_bytes = ((size_t)n_rows + 1) * (size_t)words * 4;
+    if ((e = ix->d_bm_slot.reserve(slot.size() * 4)) ||
+        (e = cudaMemcpy(ix->d_bm_slot.p, slot.data(), slot.size() * 4, cudaMemcpyHostToDevice)) ||
+        (e = cudaMemcpy(rk.p, row_key.data(), row_key.size() * 4, cudaMemcpyHostToDevice)) ||
+        (e = cudaMemcpy(mr.p, first.data(), first.size() * 4, cudaMemcpyHostToDevice)) ||
+        (e = ix->d_bm_rows.reserve(row_bytes)) || (e = cudaMemsetAsync(ix->d_bm_rows.p, 0, row_bytes, ix->stream)))
+        return give_up();
+    if (ix->codec)       // one value per object and dim: a row a list, in order
         k_bm_build_compressed<<<dim3(64, (unsigned)row_key.size()), 256, 0, ix->stream>>>(
             ix->codec, ix->dev.words, ix->dev.seg_word_off, ix->dev.key_seg, (const uint32_t *)rk.p, words,
             (uint32_t *)ix->d_bm_rows.p);
     else
         k_bm_build<<<dim3(64, (unsigned)row_key.size()), 256, 0, ix->stream>>>(
-            ix->dev.ids, ix->dev.key_off, (const uint32_t *)rk.p, words, (uint32_t *)ix->d_bm_rows.p);
+            ix->dev.ids, ix->dev.key_off, (const uint32_t *)rk.p, (const uint32_t *)mr.p,
+            ix->is_bag ? kBmMaxRows : 1u, words, (uint32_t *)ix->d_bm_rows.p);
     e = cudaGetLastError();
     if (!e) e = cudaStreamSynchronize(ix->stream);
+    if (e) return give_up();
     rk.release();
-    if (e) {
-        cudaGetLastError();
-        ix->d_bm_slot.release();
-        ix->d_bm_rows.release();
-        return false;
-    }
+    mr.release();
+    ix->bm_zero = n_rows;
     ix->bm_words = words;
     return true;
 }
@@ -236,6 +286,7 @@ DevIndex index_view(genie_index *ix, const Tuning &t) {
     d.bm_slot = bm ? (const uint32_t *)ix->d_bm_slot.p : nullptr;
     d.bm_rows = bm ? (const uint32_t *)ix->d_bm_rows.p : nullptr;
     d.bm_words = bm ? ix->bm_words : 0;
+    d.bm_zero = bm ? ix->bm_zero : 0;
     if (t.dense_bitmaps && ix->pl_tiles > 0) {
         d.planes = (const uint4 *)ix->d_planes.p;
         d.pl_row_vec = (int32_t)ix->pl_row_vec;
