@@ -34,6 +34,7 @@ constexpr uint32_t kBmMaxIds = 40 * 1024;
 constexpr uint32_t kPlTile = 16384;
 constexpr uint32_t kPlMaxItems = 255;
 constexpr uint32_t kPlMaxWeightedK = 512;
+constexpr uint32_t kPlAnyK = 128;
 // weighted queries there: items up to which a weight group is 8 (else 16), the
 // largest unit weight, and the largest bound (eleven planes)
 constexpr uint32_t kPlGroup8 = 72;
@@ -41,10 +42,16 @@ constexpr uint32_t kPlUnitMax = 31;
 constexpr uint32_t kPlBoundMax = 2047;
 // Whether a query of an index with planes is counted with them: m items that
 // end at item_end, counts of at most eight bits (one value per object and dim:
-// at most m), weighted results that fit a tile's buffer.  The plan decides by
-// it on the device, and the host by the same rule which kernels to launch.
-__host__ __device__ inline bool planes_take(int64_t m, int64_t item_end, bool weighted, uint32_t k, int32_t n_dims) {
-    return m <= (int64_t)kPlMaxItems && item_end <= 0xFFFFFFFFll && (!weighted || (k <= kPlMaxWeightedK && n_dims <= 65536));
+// at most m).  Weighted results must fit a tile's buffer, and beyond kPlAnyK
+// few of the objects may be results: a tile sums its candidates, a few times
+// k, one by one (64 queries of 8-120 items, half k = 10 and half k = 500, on
+// 20,000 objects: 209 us with lists and 328 with planes; on 500,000: 680 and
+// 602).  The plan decides by it on the device, and the host by the same rule
+// which kernels to launch.
+__host__ __device__ inline bool planes_take(int64_t m, int64_t item_end, bool weighted, uint32_t k, int32_t n_dims,
+                                            int64_t n_objects) {
+    if (m > (int64_t)kPlMaxItems || item_end > 0xFFFFFFFFll) return false;
+    return !weighted || (n_dims <= 65536 && (k <= kPlAnyK || (k <= kPlMaxWeightedK && (int64_t)k * 256 <= n_objects)));
 }
 // rows of a tile behind its keys' rows: no object, and every object
 constexpr uint32_t kPlExtraRows = 2;

@@ -110,7 +110,7 @@ __global__ void __launch_bounds__(kPlanThreads, 8) k_plan(DevIndex ix, DevQuerie
     // (1 % of the objects each) are faster there than hashed: 260,000 x 128,
     // 256 queries of 8-128 items, a quarter of them exact, 494 us before (125
     // of them hashing the exact ones) and 140 us.
-    const bool planes = ix.planes != nullptr && W.lbk != nullptr && planes_take(m, i1, weighted, k, ix.n_dims);
+    const bool planes = ix.planes != nullptr && W.lbk != nullptr && planes_take(m, i1, weighted, k, ix.n_dims, ix.n_objects);
     if (tid == 0) {
         s_total = 0;
         s_units = 0;

@@ -214,7 +214,7 @@ uint32_t launch_need(const genie_index *ix, const genie_queries *q) {
         const bool w = q->weighted && q->weight && q->weighted[i];
         const uint32_t k = q->k ? q->k[i] : q->uniform_k;
         const int64_t a = q->item_off[i], e = q->item_off[i + 1];
-        if (!planes_take(e - a, e, w, k, ix->host.n_dims)) need |= kNeedLists;
+        if (!planes_take(e - a, e, w, k, ix->host.n_dims, ix->host.n_objects)) need |= kNeedLists;
         else need |= w ? kNeedPlanesWeighted : kNeedPlanes;
     }
     return need;

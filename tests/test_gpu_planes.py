@@ -99,3 +99,14 @@ def test_more_ties_than_a_region_holds(genie, oracle):
     for wf in (None, np.ones(q, np.uint8)):
         qb = genie.QueryBatch(off, np.zeros(q, np.int32), low, low, np.full(q, k, np.uint32), w, wf)
         _check(genie, oracle, values, qb, batch=True)
+
+
+@pytest.mark.parametrize("n,k", [(20_000, 128), (20_000, 129), (131_072, 512), (131_071, 512), (131_072, 513)])
+@pytest.mark.parametrize("m", [12, 48, 49, 90])
+def test_weighted_k_and_many_candidates(genie, oracle, n, k, m):
+    """The k up to which weighted queries take the planes, and tiles whose many
+    candidates are summed a thread each (up to 48 items) or a warp four."""
+    rng = np.random.default_rng(n + k + m)
+    values = rng.integers(0, 25, size=(n, 90)).astype(np.int32)
+    qb = _queries(genie, rng, n, 90, 10, lambda i: m, lambda i: k, values, "half", 3)
+    _check(genie, oracle, values, qb)
