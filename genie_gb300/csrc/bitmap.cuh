@@ -144,6 +144,7 @@ struct BmQuery {
 
 __global__ void __launch_bounds__(kBmThreads, 1) k_bitmap(DevIndex ix, DevQueries Q, Work W, Tuning T) {
     extern __shared__ __align__(16) unsigned char smem[];
+    chain_wait();
     const uint32_t mslots = (uint32_t)T.bitmap_multi_slots;
     const BmLayout L = bm_layout(ix.n_objects, mslots);
     uint32_t *bm = (uint32_t *)(smem + L.bm);

@@ -75,6 +75,7 @@ __global__ void __launch_bounds__(kPlanThreads, 8) k_plan(DevIndex ix, DevQuerie
     __shared__ uint32_t s_inc[kPlanThreads];       // planes, weighted: the items' increments
     __shared__ unsigned long long s_groups;
     __shared__ uint32_t s_top;
+    chain_next();
     static_assert(kPlMaxItems < kPlanThreads, "one item of a planes query per thread");
     const int64_t q = blockIdx.x;
     const int64_t nq = Q.dyn ? (int64_t)Q.dyn[0] : (int64_t)Q.n_queries;
@@ -1069,6 +1070,7 @@ __device__ __forceinline__ void sparse_list(const DevIndex &ix, const DevQueries
 // drained before the next; a launch whose lists are empty costs one check.
 template <int NT>
 __global__ void __launch_bounds__(NT, NT == 512 ? 2 : 1) k_sparse(DevIndex ix, DevQueries Q, Work W, Tuning T) {
+    chain_wait();
     sparse_list<true, NT>(ix, Q, W, T);
     sparse_list<false, NT>(ix, Q, W, T);
 }
@@ -1578,6 +1580,7 @@ __device__ __forceinline__ void dense_list(const DevIndex &ix, const DevQueries 
 // Both dense work lists in one launch (1-byte and 4-byte counter tiles take
 // the same shared memory), one after the other.
 __global__ void __launch_bounds__(1024, 1) k_dense(DevIndex ix, DevQueries Q, Work W, Tuning T) {
+    chain_wait();
     dense_list<true>(ix, Q, W, T);
     dense_list<false>(ix, Q, W, T);
 }
@@ -1684,6 +1687,22 @@ int launch_plan(const DevIndex &ix, const DevQueries &Q, const Work &W, const Tu
     return 1;
 }
 
+// A kernel that starts with chain_wait, as the dependent of the one before it in the stream.
+template <class... P, class... A>
+void launch_chained(void (*kernel)(P...), int grid, int threads, size_t smem, cudaStream_t s, const A &...args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
 // The match kernels as persistent grids: the bitmap kernel, the sparse
 // kernel (both slot widths), the dense kernel (both counter widths).
 enum : int { kKernBitmap = 0, kKernSparse = 1, kKernDense = 2, kNumKern = 3 };
@@ -1719,18 +1738,19 @@ int launch_kernel(int kern, const DevIndex &ix, const DevQueries &Q, const Work 
     case kKernBitmap: {
         if (t.bitmap_bits <= 0) return 0;
         const size_t bp = bm_layout(ix.n_objects, (uint32_t)t.bitmap_multi_slots).bytes;
-        k_bitmap<<<num_sms, kBmThreads, bp, s>>>(ix, Q, W, t);
+        launch_chained(k_bitmap, num_sms, kBmThreads, bp, s, ix, Q, W, t);
         return 1;
     }
     case kKernSparse: {
         const size_t sp = sparse_smem_both(t);
-        if (t.sparse_threads == 1024) k_sparse<1024><<<grid((const void *)k_sparse<1024>, 1024, sp), 1024, sp, s>>>(ix, Q, W, t);
-        else k_sparse<512><<<grid((const void *)k_sparse<512>, 512, sp), 512, sp, s>>>(ix, Q, W, t);
+        if (t.sparse_threads == 1024)
+            launch_chained(k_sparse<1024>, grid((const void *)k_sparse<1024>, 1024, sp), 1024, sp, s, ix, Q, W, t);
+        else launch_chained(k_sparse<512>, grid((const void *)k_sparse<512>, 512, sp), 512, sp, s, ix, Q, W, t);
         return 1;
     }
     default: {
         const size_t dp = dense_smem_both(t);
-        k_dense<<<grid((const void *)k_dense, t.dense_threads, dp), t.dense_threads, dp, s>>>(ix, Q, W, t);
+        launch_chained(k_dense, grid((const void *)k_dense, t.dense_threads, dp), t.dense_threads, dp, s, ix, Q, W, t);
         return 1;
     }
     }
