@@ -280,6 +280,35 @@ struct PlCounts {
     }
 };
 
+// The sums of the block's `groups` runs of `width` threads, each of which
+// counted other items of the same objects, into the first run's planes.  buf
+// holds a vector per plane and thread.
+__device__ __forceinline__ void pl_join(PlCounts<false> &pc, uint32_t width, uint32_t groups, uint4 *buf) {
+    const uint32_t g = threadIdx.x / width;
+    for (uint32_t half = groups / 2; half > 0; half /= 2) {
+        if (g >= half && g < 2 * half) {
+#pragma unroll
+            for (int b = 0; b < 8; ++b)
+                buf[b * kPlThreads + threadIdx.x - half * width] = make_uint4(pc.c[b][0], pc.c[b][1], pc.c[b][2], pc.c[b][3]);
+        }
+        __syncthreads();
+        if (g < half) {
+            uint32_t carry[4] = {0, 0, 0, 0};
+#pragma unroll
+            for (int b = 0; b < 8; ++b) {
+                const uint4 v = buf[b * kPlThreads + threadIdx.x];
+#pragma unroll
+                for (int w = 0; w < 4; ++w) {
+                    const uint32_t x = pc.c[b][w], y = (&v.x)[w], z = carry[w];
+                    pc.c[b][w] = x ^ y ^ z;
+                    carry[w] = (x & y) | (x & z) | (y & z);
+                }
+            }
+        }
+        __syncthreads();
+    }
+}
+
 // Unit weight of the weight group starting at item u (0 past the last).
 __device__ __forceinline__ uint32_t pl_unit(const PlItems<true> &it, uint32_t u, uint32_t n, int qshift) {
     return u < n ? (it.inc[u] + ((1u << qshift) - 1u)) >> qshift : 0u;
@@ -288,13 +317,14 @@ __device__ __forceinline__ uint32_t pl_unit(const PlItems<true> &it, uint32_t u,
 // Counts of one tile over the query's items.
 template <bool WEIGHTED>
 __device__ __forceinline__ void pl_count(const unsigned char *__restrict__ tile, uint32_t mine, uint32_t n,
-                                         int qshift, const PlItems<WEIGHTED> &it, PlCounts<WEIGHTED> &pc) {
+                                         int qshift, const PlItems<WEIGHTED> &it, PlCounts<WEIGHTED> &pc,
+                                         uint32_t first = 0) {
     pc.clear();
     if constexpr (WEIGHTED) pc.unit = pl_unit(it, 0, n, qshift);
     auto load = [&](uint32_t u, uint4 (&lo)[4], uint4 (&up)[4]) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            const uint2 r = it.rows[u + i];
+            const uint2 r = it.rows[first + u + i];
             lo[i] = __ldg((const uint4 *)(tile + (r.x + mine)));
             up[i] = __ldg((const uint4 *)(tile + (r.y + mine)));
         }
@@ -332,21 +362,64 @@ __device__ __forceinline__ void pl_count(const unsigned char *__restrict__ tile,
     }
 }
 
+// Exact sums of X objects a warp, from object c of the list on: a lane every
+// 32nd item.
+template <int X>
+__device__ __forceinline__ void pl_exact_warp(const uint8_t *base, uint32_t row_bytes, uint32_t tile_lo, uint32_t c,
+                                              uint32_t n, uint32_t n_items, uint64_t lbk, const PlItems<true> &it,
+                                              PlExact &ex, PlShared &s) {
+    const uint32_t lane = lane_id();
+    const uint8_t *row[X];
+    uint32_t sum[X];
+#pragma unroll
+    for (int x = 0; x < X; ++x) {
+        row[x] = base + (uint32_t)ex.obj[min(c + x, n - 1)] * row_bytes;
+        sum[x] = 0;
+    }
+    for (uint32_t i0 = 0; i0 < n_items; i0 += 64) {
+        uint32_t v[2][X], test[2], inc[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const uint32_t i = i0 + 32 * h + lane;
+            test[h] = i < n_items ? it.test[i] : 0u;
+            inc[h] = i < n_items ? it.inc[i] : 0u;
+#pragma unroll
+            for (int x = 0; x < X; ++x) v[h][x] = __ldg(row[x] + (test[h] >> 16));
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int x = 0; x < X; ++x)
+                sum[x] += v[h][x] - ((test[h] >> 8) & 255u) <= (test[h] & 255u) ? inc[h] : 0u;
+    }
+    uint32_t mine = 0;      // lane x: object c + x's sum
+#pragma unroll
+    for (int x = 0; x < X; ++x) {
+        const uint32_t total = __reduce_add_sync(0xffffffffu, sum[x]);
+        if (lane == (uint32_t)x) mine = total;
+    }
+    if (lane < (uint32_t)X && c + lane < n) {
+        const uint64_t key = make_key(mine, tile_lo + ex.obj[c + lane]);
+        if (key >= lbk) ex.cand[atomicAdd(&s.n, 1u)] = key;
+    }
+}
+
 // Exact sums of the listed objects (x.obj[0, n), local to the tile) from the
-// objects' value rows: keys at or above lbk are appended to x.cand at s.n.  Few
-// objects, or many items: a warp sums four at a time, a lane every 32nd item.
-// Many objects (a first tile) of few items: a thread an object, whose row stays
-// in L1 while its items are read one after the other (64 queries of up to 20
-// items, k = 100, 20,000 objects: 393 us a call with a warp four, 210 so; of up
-// to 120 items 183 and 224).
+// objects' value rows: keys at or above lbk are appended to x.cand at s.n.  A
+// warp sums four objects at a time, eight when there are many (twice the loads
+// in flight).  Many objects (a first tile) of few items: a thread an object,
+// whose row stays in L1 while its items are read one after the other (64
+// queries of up to 20 items, k = 100, 20,000 objects: 393 us a call with a warp
+// four, 210 so; of up to 120 items 183 and 224).
 __device__ __forceinline__ void pl_exact(const DevIndex &ix, uint32_t tile_lo, uint32_t n, uint32_t n_items,
                                          uint64_t lbk, const PlItems<true> &it, PlExact &ex, PlShared &s) {
-    const uint32_t lane = lane_id();
-    const uint8_t *base = ix.pl_vals + (uint64_t)tile_lo * (uint64_t)ix.pl_val_row;
+    const uint32_t row_bytes = (uint32_t)ix.pl_val_row;
+    const uint8_t *base = ix.pl_vals + (uint64_t)tile_lo * (uint64_t)row_bytes;
+    constexpr uint32_t kWarps = kPlThreads / 32;
     if (n >= kPlManyExact && n_items <= kPlManyItems) {
         for (uint32_t c = threadIdx.x; c < n; c += kPlThreads) {
             const uint32_t o = ex.obj[c];
-            const uint8_t *row = base + o * (uint32_t)ix.pl_val_row;
+            const uint8_t *row = base + o * row_bytes;
             uint32_t total = 0;
 #pragma unroll 8
             for (uint32_t i = 0; i < n_items; ++i) {
@@ -356,35 +429,11 @@ __device__ __forceinline__ void pl_exact(const DevIndex &ix, uint32_t tile_lo, u
             const uint64_t key = make_key(total, tile_lo + o);
             if (key >= lbk) ex.cand[atomicAdd(&s.n, 1u)] = key;
         }
-        return;
-    }
-    for (uint32_t c = warp_id() * 4u; c < n; c += (kPlThreads / 32) * 4u) {
-        const uint8_t *row[4];
-        uint32_t sum[4] = {0, 0, 0, 0};
-#pragma unroll
-        for (int x = 0; x < 4; ++x) row[x] = base + (uint32_t)ex.obj[min(c + x, n - 1)] * (uint32_t)ix.pl_val_row;
-        for (uint32_t i0 = 0; i0 < n_items; i0 += 64) {
-            uint32_t v[2][4], test[2], inc[2];
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const uint32_t i = i0 + 32 * h + lane;
-                test[h] = i < n_items ? it.test[i] : 0u;
-                inc[h] = i < n_items ? it.inc[i] : 0u;
-#pragma unroll
-                for (int x = 0; x < 4; ++x) v[h][x] = __ldg(row[x] + (test[h] >> 16));
-            }
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-#pragma unroll
-                for (int x = 0; x < 4; ++x)
-                    sum[x] += v[h][x] - ((test[h] >> 8) & 255u) <= (test[h] & 255u) ? inc[h] : 0u;
-        }
-#pragma unroll
-        for (int x = 0; x < 4; ++x) {
-            const uint32_t total = __reduce_add_sync(0xffffffffu, sum[x]);
-            const uint64_t key = make_key(total, tile_lo + ex.obj[min(c + x, n - 1)]);
-            if (lane == 0 && c + x < n && key >= lbk) ex.cand[atomicAdd(&s.n, 1u)] = key;
-        }
+    } else if (n > 4 * kWarps) {
+        for (uint32_t c = warp_id() * 8; c < n; c += 8 * kWarps)
+            pl_exact_warp<8>(base, row_bytes, tile_lo, c, n, n_items, lbk, it, ex, s);
+    } else if (warp_id() * 4 < n) {
+        pl_exact_warp<4>(base, row_bytes, tile_lo, warp_id() * 4, n, n_items, lbk, it, ex, s);
     }
 }
 
@@ -623,7 +672,11 @@ struct PlConfig {
     static constexpr int kBlocks = WEIGHTED ? 4 : 5;        // per SM
 };
 
-template <bool WEIGHTED>
+// SPLIT: a row of a small table is shorter than the block; then runs of threads
+// count a part of the items each, and their counts are added up (1,000 x 128,
+// one query of 128 items: 49 us a call with all items in every thread, 38 so).
+// Weighted bounds need a query's items in order.
+template <bool WEIGHTED, bool SPLIT>
 __global__ void __launch_bounds__(kPlThreads, PlConfig<WEIGHTED>::kBlocks) k_planes(DevIndex ix, DevQueries Q, Work W) {
     __shared__ PlItems<WEIGHTED> items;
     __shared__ PlShared s;
@@ -635,7 +688,8 @@ __global__ void __launch_bounds__(kPlThreads, PlConfig<WEIGHTED>::kBlocks) k_pla
     const uint64_t region_k = pl_region_k(Q, W), n_work = (uint64_t)nq * (uint64_t)ix.pl_tiles;
     unsigned long long *taken = (unsigned long long *)&W.ctr[kCtrPlanes + (WEIGHTED ? 2 : 0)];
     const uint4 *entries = (const uint4 *)(W.work + (size_t)list * W.work_stride);
-    const uint32_t mine = min(tid, (uint32_t)ix.pl_row_vec - 1u) * 16u;
+    const uint32_t width = SPLIT ? next_pow2((uint32_t)ix.pl_row_vec) : kPlThreads, groups = kPlThreads / width;
+    const uint32_t mine = min(SPLIT ? tid % width : tid, (uint32_t)ix.pl_row_vec - 1u) * 16u;
     // the pair after this one is claimed while this one is counted
     unsigned long long w = 0;
     if (tid == 0) w = atomicAdd(taken, 1ull);
@@ -668,8 +722,15 @@ __global__ void __launch_bounds__(kPlThreads, PlConfig<WEIGHTED>::kBlocks) k_pla
         __syncthreads();
         if (tid == 0) w = atomicAdd(taken, 1ull);
         PlCounts<WEIGHTED> pc;
-        pl_count<WEIGHTED>((const unsigned char *)(ix.planes + (uint64_t)tile * (uint64_t)ix.pl_tile_vec), mine,
-                           pq.n_items, pq.qshift, items, pc);
+        const unsigned char *base = (const unsigned char *)(ix.planes + (uint64_t)tile * (uint64_t)ix.pl_tile_vec);
+        if constexpr (SPLIT) {
+            const uint32_t per = (pq.n_items + 8 * groups - 1) / (8 * groups) * 8;
+            const uint32_t a = min(pq.n_items, tid / width * per), e = min(pq.n_items, a + per);
+            pl_count<WEIGHTED>(base, mine, e - a, pq.qshift, items, pc, a);
+            pl_join(pc, width, groups, (uint4 *)keys.cand);
+        } else {
+            pl_count<WEIGHTED>(base, mine, pq.n_items, pq.qshift, items, pc);
+        }
         pq.region = W.scratch + (uint64_t)out_off * region_k;
         pq.cap = (uint32_t)umin64((uint64_t)pq.k * region_k, 0x7FFFFFFFull);
         if (warp_id() == 0) {

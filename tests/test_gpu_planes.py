@@ -110,3 +110,15 @@ def test_weighted_k_and_many_candidates(genie, oracle, n, k, m):
     values = rng.integers(0, 25, size=(n, 90)).astype(np.int32)
     qb = _queries(genie, rng, n, 90, 10, lambda i: m, lambda i: k, values, "half", 3)
     _check(genie, oracle, values, qb)
+
+
+@pytest.mark.parametrize("n", [1, 128, 129, 300, 4096, 8192, 8193])
+def test_small_tables_split_their_items(genie, oracle, n):
+    """Rows shorter than a block: runs of its threads count a part of the items
+    each (1 to 128 runs, some without items)."""
+    rng = np.random.default_rng(n)
+    values = rng.integers(0, 20, size=(n, 60)).astype(np.int32)
+    values[-1] = 19
+    ms = [1, 8, 9, 60, 128, 129, 254, 255]
+    qb = _queries(genie, rng, n, 60, 16, lambda i: ms[i % 8], lambda i: [1, 10, 100, 2048][i % 4], values, "", 4)
+    _check(genie, oracle, values, qb, batch=bool(n % 2))
