@@ -373,7 +373,13 @@ def measure(g, workloads, name, values, table, batch, desc, steps, warmup, strea
         if i >= 1:
             stage_tot += ms
     del bp
-    names = ["k_plan", "k_bitmap", "k_sparse", "k_dense"]
+    # the last stage counts a byte-valued plain table from its cumulative planes
+    # (k_planes reads two plane rows an item, not the posting ids), any other
+    # from counter tiles (k_dense)
+    lay = table.layout()
+    by_planes = (not table.info().codec and int(np.max(np.diff(lay["key_base"]))) <= 256 and
+                 tuning["dense_bitmaps"] > 0)
+    names = ["k_plan", "k_bitmap", "k_sparse", "k_planes" if by_planes else "k_dense"]
     # the match kernels that carry the batch (>= 15% of the match time); when
     # several share it, their posting bytes are counted over their summed time
     match_ms = stage_tot[1:]
@@ -388,6 +394,13 @@ def measure(g, workloads, name, values, table, batch, desc, steps, warmup, strea
                 "algorithmic_bytes_per_launch": alg, "peak_source": peak_kind + " (MEASURED_PEAKS.json hbm_gbs)"
                 if peak_kind == "measured" else peak_kind, "launches_timed": aux,
                 "stage_ms": {n: float(v / aux) for n, v in zip(names, stage_tot)}}
+    if by_planes:
+        # what k_planes asks of L2: two rows of a bit an object for every item
+        rows = 2.0 * n_items * ((table.i_size() + 16383) // 16384 * 2048)
+        roofline["note"] = ("achieved counts the posting bytes the queries logically touch; k_planes reads plane rows "
+                            "instead, so a fraction above 1 is bytes not read")
+        roofline["plane_row_bytes"] = rows
+        roofline["plane_row_gbs"] = rows / (dom_ms / 1e3) / 1e9
 
     # ---- e2e through the public API from host buffers.  Sequential: one
     # genie_batch_run per step (L2 flushed before each, outside the timing).

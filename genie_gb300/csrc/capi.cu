@@ -684,7 +684,12 @@ int genie_search_multi(genie_index *const *ixs, const genie_queries *qs, int32_t
         int rc = run_search(ixs[i], &qs[i], offs[i], items[i], out_ids + base[i], out_counts + base[i],
                             out_scores ? out_scores + base[i] : nullptr, false);
         if (rc) {
-            for (int32_t j = 0; j <= i; ++j) if (qs[j].n_queries && !custom[j]) ixs[j]->mu.unlock();
+            // what is in flight uses the indexes' workspaces and pinned words
+            for (int32_t j = 0; j <= i; ++j)
+                if (qs[j].n_queries && !custom[j]) {
+                    cudaStreamSynchronize(ixs[j]->stream);
+                    ixs[j]->mu.unlock();
+                }
             return rc;
         }
     }

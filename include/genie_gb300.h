@@ -255,7 +255,8 @@ typedef struct {
     int32_t sparse_load_pct;    /* posting ids per part <= this % of the hash slots */
     int32_t bitmap_bits;        /* largest id space (objects) of the bitmap kernel; -1: off */
     int32_t dense_bitmaps;      /* dense lists counted from their presence bitmaps: 1 for unweighted
-                                   queries, 2 for weighted ones, 3 both, -1 never */
+                                   queries, 2 for weighted ones, 3 both, -1 never (nor byte-valued
+                                   tables from their cumulative planes) */
 } genie_tuning;
 
 /* Batched search over one resident index: fixed-capacity device buffers,
@@ -293,8 +294,8 @@ int genie_batch_set_tuning(genie_batch *b, const genie_tuning *t);
 int genie_batch_last_stats(const genie_batch *b, int32_t *kernels, float *device_ms);
 /* Device milliseconds of each stage of the last launch of a batch created
  * with use_graph = 0: ms[0] plan (+ counter reset), ms[1] presence-bitmap
- * kernel, ms[2] sparse kernel (4- and 8-byte slots), ms[3] dense kernel
- * (1- and 4-byte counters). */
+ * kernel, ms[2] sparse kernel (4- and 8-byte slots), ms[3] planes kernels
+ * (byte-valued tables) and dense kernel (1- and 4-byte counters). */
 int genie_batch_stage_ms(const genie_batch *b, float *ms);
 
 /* ---------------------------------------------------------------- serving */
