@@ -1713,13 +1713,13 @@ int launch_planes(const DevIndex &ix, const DevQueries &Q, const Work &W, int nu
     if (!ix.planes || !W.lbk) return 0;
     int n = 0;
     if (need & kNeedPlanes) {
-        const int grid = num_sms * PlConfig<false>::kBlocks;
+        const int grid = num_sms * kPlBlocks;
         if (2u * (uint32_t)ix.pl_row_vec <= kPlThreads) k_planes<false, true><<<grid, kPlThreads, 0, s>>>(ix, Q, W);
         else k_planes<false, false><<<grid, kPlThreads, 0, s>>>(ix, Q, W);
         ++n;
     }
     if (need & kNeedPlanesWeighted) {
-        k_planes<true, false><<<num_sms * PlConfig<true>::kBlocks, kPlThreads, 0, s>>>(ix, Q, W);
+        k_planes<true, false><<<num_sms * kPlBlocks, kPlThreads, 0, s>>>(ix, Q, W);
         ++n;
     }
     if (n && ix.pl_tiles > 1) {

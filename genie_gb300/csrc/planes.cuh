@@ -48,6 +48,10 @@
 
 namespace gg {
 
+// Blocks per SM: unweighted, five (96 registers, spilled loads) take 3.75 ms for
+// the batch above and six 3.99, four 3.60; weighted, three and four take the
+// same 7.6 and five (102 registers) 13.1.
+constexpr int kPlBlocks = 4;
 constexpr uint32_t kPlThreads = 128;                   // threads that count: four warps
 constexpr uint32_t kPlTileVec = kPlThreads;            // 16-byte vectors of a full tile's row
 constexpr int kPlWSum = 11;                            // planes of a weighted bound
@@ -667,17 +671,12 @@ __device__ __forceinline__ void pl_items(const DevIndex &ix, const Work &W, int6
     }
 }
 
-template <bool WEIGHTED>
-struct PlConfig {
-    static constexpr int kBlocks = WEIGHTED ? 4 : 5;        // per SM
-};
-
 // SPLIT: a row of a small table is shorter than the block; then runs of threads
 // count a part of the items each, and their counts are added up (1,000 x 128,
 // one query of 128 items: 49 us a call with all items in every thread, 38 so).
 // Weighted bounds need a query's items in order.
 template <bool WEIGHTED, bool SPLIT>
-__global__ void __launch_bounds__(kPlThreads, PlConfig<WEIGHTED>::kBlocks) k_planes(DevIndex ix, DevQueries Q, Work W) {
+__global__ void __launch_bounds__(kPlThreads, kPlBlocks) k_planes(DevIndex ix, DevQueries Q, Work W) {
     __shared__ PlItems<WEIGHTED> items;
     __shared__ PlShared s;
     __shared__ typename PlScratch<WEIGHTED>::type keys;
