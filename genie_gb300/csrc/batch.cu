@@ -77,6 +77,11 @@ DevQueries device_queries(const genie_batch *b) {
 
 int enqueue(genie_batch *b, cudaStream_t s) {
     DeviceContext &ctx = device_context(b->ix->device);
+    const bool planes = b->ix->pl_tiles > 0 && b->tuning.dense_bitmaps;
+    if (b->graph_valid && b->cfg.use_graph && b->graph_planes == planes && (!planes || b->graph_need == b->need)) {
+        cudaError_t e = cudaGraphLaunch(b->gexec, s);
+        return e ? cuda_fail(e, "graph launch") : GENIE_OK;
+    }
     const DevQueries q = device_queries(b);
     const DevIndex d = index_view(b->ix, b->tuning);     // directories built before a capture
     if (d.planes && !b->ws.planes.p) {                   // earlier launches may still use the scratch

@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cmath>
 #include <cstdint>
 #include <mutex>
@@ -123,9 +124,10 @@ struct genie_index {
     uint32_t bm_zero = 0;
     gg::DevBuf d_bm_slot, d_bm_rows;
     std::vector<std::pair<int32_t, gg::DevBuf *>> dirs;
-    int64_t pl_bytes = -1;           // what the planes take (0: the index has none, -1: not looked at)
+    std::atomic<int64_t> pl_bytes{-1};   // what the planes take (0: the index has none, -1: not looked at)
     int64_t pl_touched = 0;          // posting ids its searches have touched before they were built
-    int64_t pl_tiles = 0, pl_row_vec = 0;      // set once built
+    std::atomic<int64_t> pl_tiles{0};    // set once built
+    int64_t pl_row_vec = 0;
     gg::DevBuf d_planes, d_pl_vals;
     cudaStream_t stream = nullptr;
     std::mutex mu;                   // serialises searches on this handle's workspace

@@ -177,7 +177,7 @@ bool build(genie_index *ix) {
     const int64_t n = h.n_objects, nk = h.n_keys();
     const int64_t tiles = (n + kPlTile - 1) / kPlTile;
     const int64_t row_vec = tiles > 1 ? (int64_t)kPlTile / 128 : (n + 127) / 128, rows = nk + kPlExtraRows;
-    const size_t bytes = (size_t)ix->pl_bytes;
+    const size_t bytes = (size_t)ix->pl_bytes.load();
     const int32_t dims_at_once = (int32_t)std::min<int64_t>(h.n_dims, std::max<int64_t>(1, (int64_t)kPlColumnBytes / n));
     const int32_t val_row = (h.n_dims + 15) & ~15;
     size_t free_b = 0, total_b = 0;
@@ -244,6 +244,7 @@ bool build(genie_index *ix) {
 // much: a table searched once or twice never pays for them, and none pays more
 // than about twice what it would have.  Past that point nothing is counted.
 void note_search(genie_index *ix, const genie_queries *q) {
+    if (ix->pl_bytes == 0 || ix->pl_tiles > 0) return;
     std::lock_guard<std::mutex> g(ix->dir_mu);
     if (ix->pl_bytes < 0) ix->pl_bytes = planes_bytes(ix);
     if (ix->pl_bytes == 0 || ix->pl_tiles > 0) return;
@@ -259,6 +260,7 @@ void note_search(genie_index *ix, const genie_queries *q) {
 }
 
 uint32_t launch_need(const genie_index *ix, const genie_queries *q) {
+    if (ix->pl_bytes == 0) return kNeedLists;          // never any planes
     uint32_t need = 0;
     for (int64_t i = 0; i < q->n_queries; ++i) {
         const bool w = q->weighted && q->weight && q->weighted[i];
