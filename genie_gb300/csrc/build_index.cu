@@ -352,6 +352,7 @@ int build_device_index(const int32_t *values, int64_t n, int32_t d, genie_index 
     h.n_objects = n;
     h.n_dims = d;
     h.mult_max = 1;
+    h.whole = true;
     h.dim_min.assign(bounds.begin(), bounds.begin() + d);
     h.dim_max.assign(bounds.begin() + d, bounds.end());
     std::vector<DimPlan> plan((size_t)d);

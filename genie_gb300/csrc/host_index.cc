@@ -64,6 +64,7 @@ bool build_host_index(const int32_t *values, int64_t n, int32_t d, HostIndex &ix
         for (int64_t i = 0; i < n; ++i) dst[pos[(size_t)(values[i * d + j] - mn)]++] = (uint32_t)i;
     });
     ix.key_off[ix.n_keys()] = n * d;
+    ix.whole = true;
     return true;
 }
 
@@ -91,16 +92,44 @@ bool build_host_index_bag(const int32_t *values, const int64_t *row_off, int64_t
     for (int64_t r = 0; r < n; ++r)
         for (int64_t t = row_off[r]; t < row_off[r + 1]; ++t) ix.ids[pos[(size_t)(values[t] - mn)]++] = (uint32_t)r;
     // a row repeating a value repeats its id in that list (adjacent entries)
+    ix.mult_max = most_repeats(ix);
+    return true;
+}
+
+int32_t most_repeats(const HostIndex &ix) {
     int32_t best = 1;
-    for (int64_t v = 0; v < nk; ++v) {
+    for (int64_t v = 0; v < ix.n_keys(); ++v) {
         int32_t run = 1;
         for (int64_t p = ix.key_off[v] + 1; p < ix.key_off[v + 1]; ++p) {
             run = ix.ids[p] == ix.ids[p - 1] ? run + 1 : 1;
             best = std::max(best, run);
         }
     }
-    ix.mult_max = best;
-    return true;
+    return best;
+}
+
+bool lists_every_object_once(const HostIndex &ix) {
+    const int64_t n = ix.n_objects;
+    for (int32_t d = 0; d < ix.n_dims; ++d) {
+        const int64_t width = (int64_t)ix.dim_max[d] - ix.dim_min[d] + 1;
+        const int64_t a = ix.key_base[d], e = ix.key_base[d + 1];
+        if (width <= 0 || e - a != width || ix.key_off[e] - ix.key_off[a] != n) return false;
+    }
+    // n ids a dim, so every object is listed once when none is listed twice
+    std::atomic_bool once{true};
+    parallel_for(ix.n_dims, [&](int64_t d) {
+        if (!once) return;
+        std::vector<bool> seen((size_t)n, false);
+        const int64_t a = ix.key_off[ix.key_base[d]];
+        for (int64_t p = a; p < a + n; ++p) {
+            if (seen[ix.ids[(size_t)p]]) {
+                once = false;
+                return;
+            }
+            seen[ix.ids[(size_t)p]] = true;
+        }
+    });
+    return once;
 }
 
 bool item_span(const HostIndex &ix, int32_t dim, int32_t low, int32_t up, int64_t &start, int64_t &end) {

@@ -155,7 +155,15 @@ int load_index(const char *path, genie_index *ix) {
         }
     }
     ix->is_bag = (flags & 1u) != 0;
-    if (!ix->codec) return upload_index(ix);
+    if (!ix->codec) {
+        // lists that repeat an id are a bag's, whatever the flags say: their
+        // bitmaps take a row a listing and their counts go past the items'
+        const int32_t repeats = most_repeats(h);
+        if (repeats > 1) ix->is_bag = true;
+        if (repeats > h.mult_max) h.mult_max = repeats;
+        h.whole = !ix->is_bag && lists_every_object_once(h);
+        return upload_index(ix);
+    }
     return upload_compressed(ix, words, key_seg, seg_word_off, seg_first, seg_len);
 }
 

@@ -159,11 +159,14 @@ __global__ void k_pl_ends(uint4 *planes, int64_t tiles, int64_t keys, int64_t ro
     }
 }
 
-// Bytes of the index's planes; 0 when it has none.
+// Bytes of the index's planes; 0 when it has none.  Planes stand for one value
+// per object and dim: an index from a file whose dims miss an object, list one
+// twice, or hold lists outside their value range has none (k_pl_columns would
+// leave a byte of a missing object unset, and k_pl_build index by it).
 int64_t planes_bytes(const genie_index *ix) {
     const HostIndex &h = ix->host;
     const int64_t n = h.n_objects, nk = h.n_keys();
-    if (ix->is_bag || ix->sub_shift >= 0 || ix->codec || n <= 0 || nk <= 0) return 0;
+    if (!h.whole || ix->is_bag || ix->sub_shift >= 0 || ix->codec || n <= 0 || nk <= 0) return 0;
     for (int32_t j = 0; j < h.n_dims; ++j)
         if (h.key_base[j + 1] - h.key_base[j] > kPlMaxValues) return 0;
     const int64_t tiles = (n + kPlTile - 1) / kPlTile;
