@@ -75,36 +75,41 @@ DevQueries device_queries(const genie_batch *b) {
     return q;
 }
 
+bool caller_captures(const genie_batch *b, cudaStream_t s) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (s != b->stream) cudaStreamIsCapturing(s, &status);
+    return status != cudaStreamCaptureStatusNone;
+}
+
 int enqueue(genie_batch *b, cudaStream_t s) {
     DeviceContext &ctx = device_context(b->ix->device);
-    const bool planes = b->ix->pl_tiles > 0 && b->tuning.dense_bitmaps;
-    if (b->graph_valid && b->cfg.use_graph && b->graph_planes == planes && (!planes || b->graph_need == b->need)) {
+    const bool planes = b->ix->pl_tiles > 0 && b->tuning.dense_bitmaps && b->ws.planes.p;
+    // A caller that captures a launch replays it for whatever it stages later:
+    // no kernel is left out.
+    const bool captured = caller_captures(b, s);
+    const uint32_t need = captured ? (uint32_t)kNeedAll : b->need;
+    if (b->graph_valid && b->cfg.use_graph && b->graph_planes == planes && (!planes || b->graph_need == need)) {
         cudaError_t e = cudaGraphLaunch(b->gexec, s);
         return e ? cuda_fail(e, "graph launch") : GENIE_OK;
     }
     const DevQueries q = device_queries(b);
-    const DevIndex d = index_view(b->ix, b->tuning);     // directories built before a capture
-    if (d.planes && !b->ws.planes.p) {                   // earlier launches may still use the scratch
-        cudaError_t e = cudaDeviceSynchronize();
-        if (!e) e = b->ws.reserve_planes(b->cfg.max_queries);
-        if (e) return cuda_fail(e, "batch buffers");
-        b->graph_valid = false;
-    }
+    DevIndex d = index_view(b->ix, b->tuning);           // directories built before a capture
+    if (!planes) d.planes = nullptr;
     const Work w = b->ws.view(b->cfg.max_queries, true);
     if (!b->cfg.use_graph) {
         // direct launches, with an event after every stage for per-kernel timing
-        b->last_kernels = launch_match(d, q, w, b->tuning, ctx.num_sms, s, b->stage_ev, b->need);
+        b->last_kernels = launch_match(d, q, w, b->tuning, ctx.num_sms, s, captured ? nullptr : b->stage_ev, need);
         cudaError_t e = cudaGetLastError();
         return e ? cuda_fail(e, "batch launch") : GENIE_OK;
     }
-    if (!b->graph_valid || b->graph_planes != (d.planes != nullptr) || (d.planes && b->graph_need != b->need)) {
+    if (!b->graph_valid || b->graph_planes != (d.planes != nullptr) || (d.planes && b->graph_need != need)) {
         b->graph_valid = false;
         if (b->gexec) cudaGraphExecDestroy(b->gexec);
         b->gexec = nullptr;
         cudaGraph_t g = nullptr;
         cudaError_t e = cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal);
         if (e) return cuda_fail(e, "graph capture");
-        b->last_kernels = launch_match(d, q, w, b->tuning, ctx.num_sms, b->stream, nullptr, b->need);
+        b->last_kernels = launch_match(d, q, w, b->tuning, ctx.num_sms, b->stream, nullptr, need);
         cudaError_t le = cudaGetLastError();
         e = cudaStreamEndCapture(b->stream, &g);
         if (le) {
@@ -117,7 +122,7 @@ int enqueue(genie_batch *b, cudaStream_t s) {
         if (e) return cuda_fail(e, "graph instantiate");
         b->graph_valid = true;
         b->graph_planes = d.planes != nullptr;
-        b->graph_need = b->need;
+        b->graph_need = need;
     }
     cudaError_t e = cudaGraphLaunch(b->gexec, s);
     return e ? cuda_fail(e, "graph launch") : GENIE_OK;
@@ -254,6 +259,13 @@ int genie_batch_create(genie_index *ix, const genie_batch_config *cfg, genie_bat
     b->tuning = ix->tuning;
     const int64_t Q = cfg->max_queries, I = cfg->max_items > 0 ? cfg->max_items : 1, K = (int64_t)Q * cfg->max_k;
     const int64_t U = cfg->max_units > 0 ? cfg->max_units : 16 * I;
+    // what the planes need is there before they are: a launch allocates nothing
+    // and every launch of a batch, also one its caller captured, uses the same
+    // buffers.  Without the memory for it the batch stays on the lists.
+    if (may_have_planes(ix) && b->ws.reserve_planes(Q)) {
+        cudaGetLastError();
+        b->ws.planes.release();
+    }
     cudaError_t e = b->ws.reserve(Q, I, U, K);
     if (!e) e = b->dyn.reserve(16);
     if (!e) e = cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking);
@@ -291,6 +303,7 @@ int genie_batch_launch(genie_batch *b, void *stream) {
     if (!b) return fail(GENIE_ERR_INVALID_ARG, "batch is NULL");
     cudaSetDevice(b->ix->device);
     cudaStream_t s = stream ? (cudaStream_t)stream : b->stream;
+    if (caller_captures(b, s)) return enqueue(b, s);      // nothing runs yet that the events could time
     cudaEventRecord(b->ev0, s);
     int rc = enqueue(b, s);
     cudaEventRecord(b->ev1, s);

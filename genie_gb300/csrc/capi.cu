@@ -337,6 +337,12 @@ int run_search(genie_index *ix, const genie_queries *q, const std::vector<int64_
     const size_t o_ids = place((size_t)sumk * 4), o_counts = place((size_t)sumk * 4);
     const size_t o_scores = place(out_scores ? (size_t)sumk * 4 : 0);
     const bool small = at <= kCallBytes && ix->host_err != nullptr;
+    DevIndex d = index_view(ix, ix->tuning);
+    if (d.planes && ws.reserve_planes(Q)) {     // no room: on the lists
+        cudaGetLastError();
+        ws.planes.release();
+        d.planes = nullptr;
+    }
     cudaError_t e = ws.reserve(Q, n_items, count_units(ix->host, q), sumk, !small);
     if (!e && small) e = ws.call.reserve(kCallBytes);
     if (e) return cuda_fail(e, "search workspace");
@@ -390,8 +396,6 @@ int run_search(genie_index *ix, const genie_queries *q, const std::vector<int64_
         dq.out_off = (const int64_t *)ws.out_off.p;
     }
     DeviceContext &ctx = device_context(ix->device);
-    const DevIndex d = index_view(ix, ix->tuning);
-    if (d.planes && (e = ws.reserve_planes(Q))) return cuda_fail(e, "search workspace");
     Work w = ws.view(Q, out_scores != nullptr);
     if (small) {
         w.ctr = (uint32_t *)(dev + o_ctr);

@@ -49,7 +49,8 @@ struct Workspace {
     int64_t done_q = 0;
     // io: the query inputs and results too (a small call has its own, `call`)
     cudaError_t reserve(int64_t Q, int64_t items, int64_t units, int64_t sumk, bool io = true);
-    // what a search with an index's planes needs beside; before view()
+    // what a search with an index's planes needs beside; before reserve() and
+    // view() (when it fails it may have freed the scratch)
     cudaError_t reserve_planes(int64_t Q);
     void release();
     Work view(int64_t Q, bool scores) const;
@@ -70,6 +71,8 @@ DevIndex index_view(genie_index *ix, const Tuning &t);
 // cumulative planes of a byte-valued index (planes.cu) once its searches are
 // worth them.
 void note_search(genie_index *ix, const genie_queries *q);
+// Whether the index's values allow planes, built or not.
+bool may_have_planes(genie_index *ix);
 // Kernels that a batch may need on an index with planes (LaunchNeed); a batch
 // without them needs kNeedLists.
 uint32_t launch_need(const genie_index *ix, const genie_queries *q);

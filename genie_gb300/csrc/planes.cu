@@ -262,6 +262,12 @@ void note_search(genie_index *ix, const genie_queries *q) {
     if (ix->pl_touched >= enough && !build(ix)) ix->pl_bytes = 0;
 }
 
+bool may_have_planes(genie_index *ix) {
+    std::lock_guard<std::mutex> g(ix->dir_mu);
+    if (ix->pl_bytes < 0) ix->pl_bytes = planes_bytes(ix);
+    return ix->pl_bytes > 0;
+}
+
 uint32_t launch_need(const genie_index *ix, const genie_queries *q) {
     if (ix->pl_bytes == 0) return kNeedLists;          // never any planes
     uint32_t need = 0;
