@@ -141,7 +141,7 @@ int stage_async(genie_batch *b, const genie_queries *q, cudaStream_t s) {
         const uint32_t k = q->k ? q->k[i] : q->uniform_k;
         if (k > b->cfg.max_k) return fail(GENIE_ERR_INVALID_ARG, "k=%u exceeds the batch capacity %u", k, b->cfg.max_k);
     }
-    note_search(b->ix, q);
+    note_search(b->ix, q, b->tuning);
     b->need |= launch_need(b->ix, q);
     // The caller's item arrays are uploaded from where they are: a copy from
     // pageable memory returns once the source may be reused, and on a

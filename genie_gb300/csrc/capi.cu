@@ -314,7 +314,7 @@ int run_search(genie_index *ix, const genie_queries *q, const std::vector<int64_
     if (ix->sub_shift >= 0) return subseq_search(ix, q, out_off, n_items, out_ids, out_counts, out_scores, sync);
     const int64_t Q = q->n_queries;
     const int64_t sumk = out_off[Q];
-    note_search(ix, q);
+    note_search(ix, q, ix->tuning);
     Workspace &ws = ix->ws;
     const bool has_w = q->weighted && q->weight;
     // A small call is packed: inputs and zeroed counters in one upload, error

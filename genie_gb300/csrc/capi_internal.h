@@ -67,10 +67,10 @@ int validate_queries(const genie_queries *q, std::vector<int64_t> &out_off, int6
 // The device view of an index for a tuning: ix->dev plus the tile
 // directories of the tuning's two tile sizes (built on first use).
 DevIndex index_view(genie_index *ix, const Tuning &t);
-// Called with every batch of queries before it is searched: builds the
-// cumulative planes of a byte-valued index (planes.cu) once its searches are
-// worth them.
-void note_search(genie_index *ix, const genie_queries *q);
+// Called with every batch of queries before it is searched with a tuning:
+// builds the cumulative planes of a byte-valued index (planes.cu) once the
+// searches that may use them are worth it.
+void note_search(genie_index *ix, const genie_queries *q, const Tuning &t);
 // Whether the index's values allow planes, built or not.
 bool may_have_planes(genie_index *ix);
 // Kernels that a batch may need on an index with planes (LaunchNeed); a batch

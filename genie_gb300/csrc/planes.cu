@@ -7,7 +7,8 @@
 // them).  A plane row is n_objects / 8 bytes against 4 bytes a posting id, so
 // the planes take (values per dim) / 32 times the ids' bytes: eight times for
 // 256 values.  They are built when a quarter of the device memory that is free
-// then holds them, once per index (note_search), and kept while it lives.  The
+// then holds all that is kept, once per index (note_search), and kept while it
+// lives.  The
 // values themselves are kept too, one byte each, object by object (a 32nd of
 // 256 planes): a weighted tile sums its few candidates from them, whose bytes
 // of one object lie in one or two lines, where the planes would cost a line
@@ -188,20 +189,22 @@ bool build(genie_index *ix) {
         cudaGetLastError();
         return false;
     }
-    if (bytes > free_b / 4) return false;
+    const size_t val_bytes = (size_t)n * (size_t)val_row, col_bytes = (size_t)dims_at_once * (size_t)n;
+    if (bytes + val_bytes > free_b / 4 || bytes + val_bytes + col_bytes > free_b / 2) return false;
     static_assert(kPlMaxValues * kPlSubWords * 4 == 65536, "shared presence bits");
     DevBuf col;
     cudaError_t e;
     if ((e = cudaFuncSetAttribute((const void *)k_pl_build, cudaFuncAttributeMaxDynamicSharedMemorySize, 65536)) ||
         (e = cudaFuncSetAttribute((const void *)k_pl_columns, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPlSpan)) ||
         (e = cudaMalloc(&ix->d_planes.p, bytes)) ||
-        (e = ix->d_pl_vals.reserve((size_t)n * (size_t)val_row)) || (e = cudaMalloc(&col.p, (size_t)dims_at_once * (size_t)n))) {
+        (e = cudaMalloc(&ix->d_pl_vals.p, val_bytes)) || (e = cudaMalloc(&col.p, col_bytes))) {
         cudaGetLastError();
         ix->d_planes.release();
         ix->d_pl_vals.release();
         return false;
     }
     ix->d_planes.bytes = bytes;
+    ix->d_pl_vals.bytes = val_bytes;
     const uint32_t subs = (uint32_t)((row_vec * 4 + kPlSubWords - 1) / kPlSubWords);
     for (int32_t d0 = 0; d0 < h.n_dims; d0 += dims_at_once) {
         const int32_t nd = std::min(dims_at_once, h.n_dims - d0);
@@ -246,8 +249,9 @@ bool build(genie_index *ix) {
 // in 45 ms), so they are built when the index's searches have touched that
 // much: a table searched once or twice never pays for them, and none pays more
 // than about twice what it would have.  Past that point nothing is counted.
-void note_search(genie_index *ix, const genie_queries *q) {
-    if (ix->pl_bytes == 0 || ix->pl_tiles > 0) return;
+// Searches whose tuning keeps them off the planes do not count.
+void note_search(genie_index *ix, const genie_queries *q, const Tuning &t) {
+    if (!t.dense_bitmaps || ix->pl_bytes == 0 || ix->pl_tiles > 0) return;
     std::lock_guard<std::mutex> g(ix->dir_mu);
     if (ix->pl_bytes < 0) ix->pl_bytes = planes_bytes(ix);
     if (ix->pl_bytes == 0 || ix->pl_tiles > 0) return;

@@ -1,0 +1,52 @@
+"""Which kernels a search launches: the planes of a byte-valued table, built and
+used when and only when they should be.  A table of one tile shows it by the
+launches of an unweighted batch: the plan and one planes kernel, against the
+plan and the three list kernels."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+PLANES, LISTS = 2, 4
+
+
+def _table(genie, n=5_000, d=24, width=60, seed=1):
+    values = np.random.default_rng(seed).integers(0, width, size=(n, d)).astype(np.int32)
+    values[0], values[1] = 0, width - 1
+    return genie.Table.from_values(values), values
+
+
+def _exact(genie, values, q, m, k=10, seed=2, weighted=False):
+    rng = np.random.default_rng(seed)
+    n, d = values.shape
+    dim = np.concatenate([rng.choice(d, m, replace=m > d) for _ in range(q)]).astype(np.int32)
+    low = values[np.repeat(rng.integers(0, n, q), m), dim]
+    w = rng.uniform(0.5, 2.0, q * m).astype(np.float32) if weighted else None
+    return genie.QueryBatch(np.arange(q + 1) * m, dim, low, low, k, w, np.ones(q, np.uint8) if weighted else None)
+
+
+def _wide(genie, table, times=1):
+    """Searches that touch `times` as many posting ids as the planes have bytes."""
+    lay = table.layout()
+    d, n = len(lay["dim_min"]), table.info().n_objects
+    tiles = -(-n // 16384)
+    row = 2048 if tiles > 1 else 16 * -(-n // 128)
+    q = 1 + int(times * tiles * row * (len(lay["key_offsets"]) + 1) / (n * d))
+    lo, up = int(lay["dim_min"].min()), int(lay["dim_max"].max())
+    return genie.QueryBatch(np.arange(q + 1) * d, np.tile(np.arange(d), q), np.full(q * d, lo), np.full(q * d, up), 1)
+
+
+def test_searches_off_the_planes_do_not_build_them(genie):
+    table, values = _table(genie)
+    wide, few = _wide(genie, table, 3), _exact(genie, values, 1, 2)
+    off = genie.Batch(table, wide.n_queries, len(wide.dim), 1, max_units=len(wide.dim) * 61)
+    off.set_tuning(dense_bitmaps=-1)
+    off.run(wide)
+    on = genie.Batch(table, 1, 2, 10)
+    on.run(few)
+    assert on.last_stats()[0] == LISTS
+    genie.search(table, wide)
+    on.run(few)
+    assert on.last_stats()[0] == PLANES
+    off.run(wide)
+    assert off.last_stats()[0] == LISTS
