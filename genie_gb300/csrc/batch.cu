@@ -385,8 +385,10 @@ int genie_batch_stage_ms(const genie_batch *b, float *ms) {
 
 // Times each candidate shape on the sample (one warm-up, three timed graph
 // launches) and keeps the fastest.  Candidates vary the hash slots per CTA
-// (hence CTAs per SM), the dense tile, the sparse/dense crossover and the
-// presence-bitmap kernel (on with a bitmap size, or off).
+// (hence CTAs per SM), the dense tile, the sparse/dense crossover, the
+// presence-bitmap kernel (on with a bitmap size, or off) and the dense lists'
+// bitmaps (on or off; always on for a table that may have planes: off keeps the
+// batch off those too, whereas the sample is timed on whatever exists by then).
 int genie_batch_autotune(genie_batch *b, const genie_queries *sample, genie_tuning *chosen) {
     if (!b || !sample) return fail(GENIE_ERR_INVALID_ARG, "NULL argument");
     cudaSetDevice(b->ix->device);
@@ -433,6 +435,7 @@ int genie_batch_autotune(genie_batch *b, const genie_queries *sample, genie_tuni
         return GENIE_OK;
     };
     for (const Cand &c : cands) {
+        if (c.dbm < 0 && may_have_planes(b->ix)) continue;
         genie_tuning t{};
         t.sparse_slots = c.slots;
         t.sparse_ctas_per_sm = c.ctas;

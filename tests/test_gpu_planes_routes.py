@@ -50,3 +50,15 @@ def test_searches_off_the_planes_do_not_build_them(genie):
     assert on.last_stats()[0] == PLANES
     off.run(wide)
     assert off.last_stats()[0] == LISTS
+
+
+@pytest.mark.parametrize("weighted", [False, True])
+def test_autotuning_keeps_the_planes(genie, weighted):
+    """Tuned before the planes exist, a batch uses them when they do."""
+    table, values = _table(genie)
+    sample = _exact(genie, values, 4, 3, weighted=weighted)
+    b = genie.Batch(table, 4, 12, 10)
+    assert b.autotune(sample)["dense_bitmaps"] > 0
+    genie.search(table, _wide(genie, table))
+    b.run(sample)
+    assert b.last_stats()[0] == PLANES
