@@ -75,10 +75,13 @@ struct PlExact {
     uint64_t cand[kPlCand];
     uint16_t obj[kPlCand];
 };
-// The keys of a table of one tile, which need no merge.
+// The keys of a table of one tile, which need no merge; before there are any,
+// the counts that pl_join adds up, in 16-byte vectors.
 struct PlKeys {
-    uint64_t cand[kCandCap];
+    alignas(16) uint64_t cand[kCandCap];
 };
+static_assert(alignof(PlKeys) % sizeof(uint4) == 0, "pl_join's vectors are aligned");
+static_assert(sizeof(PlKeys::cand) >= 8 * kPlThreads * sizeof(uint4), "eight planes of every thread");
 // A tile's keys in shared memory: exact keys of a weighted one, the result of
 // an unweighted query of a table of one tile.
 template <bool WEIGHTED>
@@ -726,7 +729,7 @@ __global__ void __launch_bounds__(kPlThreads, kPlBlocks) k_planes(DevIndex ix, D
             const uint32_t per = (pq.n_items + 8 * groups - 1) / (8 * groups) * 8;
             const uint32_t a = min(pq.n_items, tid / width * per), e = min(pq.n_items, a + per);
             pl_count<WEIGHTED>(base, mine, e - a, pq.qshift, items, pc, a);
-            pl_join(pc, width, groups, (uint4 *)keys.cand);
+            pl_join(pc, width, groups, reinterpret_cast<uint4 *>(keys.cand));
         } else {
             pl_count<WEIGHTED>(base, mine, pq.n_items, pq.qshift, items, pc);
         }
