@@ -346,7 +346,7 @@ int genie_batch_get_tuning(const genie_batch *b, genie_tuning *out) {
 int genie_batch_set_tuning(genie_batch *b, const genie_tuning *t) {
     if (!b || !t) return fail(GENIE_ERR_INVALID_ARG, "NULL argument");
     Tuning r = from_public(b->tuning, *t);
-    const size_t smem_cap = 227 * 1024 - 64;     // dynamic + the kernels' static words
+    const size_t smem_cap = kSmemCap;
     if (r.sparse_slots_packed < 1024 || sparse_smem_bytes(r, true) > smem_cap ||
         sparse_smem_bytes(r, false) > smem_cap || r.dense_tile_u8 < 4096 ||
         dense_smem_bytes(r, true) > smem_cap || dense_smem_bytes(r, false) > smem_cap ||

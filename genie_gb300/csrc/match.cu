@@ -1274,6 +1274,15 @@ __device__ __forceinline__ void bitmap_counts(const uint32_t *__restrict__ rows,
 // query part, keeping its running top-k.  Replaces the per-query global bitmap
 // (match.cu:276-294, match_device_utils.h:422-446), which wraps above
 // 2^bits - 1; these counters are sized from the item count and never wrap.
+// Beside the counters the tile's keys, candidates and staged units; and, where
+// that leaves room, the start of each unit's list, which a part of several
+// tiles otherwise reads again in every tile.
+constexpr size_t kDenseFixed = (size_t)kMaxK * 8 + (size_t)kCandCap * 8 + kItemChunk * 28 + 16 + sizeof(SelectScratch) +
+                               kItemChunk * 12 + 64;
+__host__ __device__ constexpr bool dense_keeps_starts(size_t counter_bytes) {
+    return counter_bytes + kDenseFixed + kItemChunk * 8 <= kSmemCap;
+}
+
 template <bool SMALL>
 __device__ __forceinline__ void dense_list(const DevIndex &ix, const DevQueries &Q, const Work &W, const Tuning &T) {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -1297,6 +1306,7 @@ __device__ __forceinline__ void dense_list(const DevIndex &ix, const DevQueries 
     uint32_t *bm_inc = bm_row + kItemChunk;
     uint32_t *unit_bm = bm_inc + kItemChunk;
     // and where its list starts
+    const bool keep_s0 = dense_keeps_starts(cnt_bytes);
     int64_t *unit_s0 = (int64_t *)(unit_bm + kItemChunk);
     __shared__ uint32_t s_q, s_p, s_nS, s_nc, s_L, s_nbm, s_fit;
 
@@ -1338,7 +1348,7 @@ __device__ __forceinline__ void dense_list(const DevIndex &ix, const DevQueries 
         if (single && (int32_t)tid < qi.n_units) {
             const int64_t it = qi.unit0 + tid;
             const int64_t s0 = W.span_start[it], e0 = s0 + W.span_len[it];
-            unit_s0[tid] = s0;
+            if (keep_s0) unit_s0[tid] = s0;
             st.inc[tid] = W.inc[it];
             uint32_t bm = (use_bm && e0 > s0) ? ix.bm_slot[W.unit_key[it]] : 0xFFFFFFFFu;
             // more rows than a chunk holds: the rest of the lists keep to their
@@ -1369,7 +1379,7 @@ __device__ __forceinline__ void dense_list(const DevIndex &ix, const DevQueries 
                 uint32_t len = 0;
                 if ((int32_t)tid < mc) {
                     const int64_t it = qi.unit0 + c0 + tid;
-                    const int64_t s0 = single ? unit_s0[tid] : W.span_start[it];
+                    const int64_t s0 = single && keep_s0 ? unit_s0[tid] : W.span_start[it];
                     auto e0 = [&] { return s0 + W.span_len[it]; };
                     const uint32_t inc = single ? st.inc[tid] : W.inc[it];
                     uint32_t row = 0xFFFFFFFFu;
@@ -1594,9 +1604,8 @@ size_t sparse_smem_bytes(const Tuning &t, bool packed) {
 }
 
 size_t dense_smem_bytes(const Tuning &t, bool small) {
-    size_t c = (size_t)(small ? t.dense_tile_u8 : t.dense_tile_u32 * 4);
-    return c + (size_t)kMaxK * 8 + (size_t)kCandCap * 8 + kItemChunk * 28 + 16 + sizeof(SelectScratch) + kItemChunk * 12 +
-           kItemChunk * 8 + 64;
+    const size_t c = (size_t)(small ? t.dense_tile_u8 : t.dense_tile_u32 * 4);
+    return c + kDenseFixed + (dense_keeps_starts(c) ? kItemChunk * 8 : 0);
 }
 
 Tuning default_tuning() {

@@ -12,6 +12,8 @@ Tuning default_tuning();
 void read_oob(unsigned long long out[4]);
 size_t sparse_smem_bytes(const Tuning &t, bool packed);
 size_t dense_smem_bytes(const Tuning &t, bool small);
+// Dynamic shared memory a kernel may have beside its static words.
+constexpr size_t kSmemCap = 227 * 1024 - 64;
 cudaError_t prepare_kernels(const Tuning &t);
 // Allow the largest dynamic shared memory on every match kernel (once per device).
 cudaError_t prepare_kernels_max();
