@@ -1283,6 +1283,16 @@ __host__ __device__ constexpr bool dense_keeps_starts(size_t counter_bytes) {
     return counter_bytes + kDenseFixed + kItemChunk * 8 <= kSmemCap;
 }
 
+// Tiles that may count lists from their bitmaps: the byte counters take whole
+// vectors of 128 objects, the 4-byte counters words of 32.
+__host__ __device__ constexpr bool dense_tile_takes_bitmaps(uint32_t tile, bool small) {
+    return tile % (small ? 128u : 32u) == 0;
+}
+// every tile that genie_batch_set_tuning makes of a dense_tile (multiples of
+// 256, a quarter of it rounded to 64) does
+static_assert(dense_tile_takes_bitmaps(4096 + 256, true) && dense_tile_takes_bitmaps(10048, false) &&
+                  dense_tile_takes_bitmaps(1024 + 64, false), "bitmaps in tiles of every tuning");
+
 template <bool SMALL>
 __device__ __forceinline__ void dense_list(const DevIndex &ix, const DevQueries &Q, const Work &W, const Tuning &T) {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -1316,8 +1326,8 @@ __device__ __forceinline__ void dense_list(const DevIndex &ix, const DevQueries 
     const uint32_t *dir = SMALL ? ix.dir8 : ix.dir32;
     const bool use_dir = dir != nullptr && ix.dir_slot != nullptr && W.unit_key != nullptr &&
                          (SMALL ? ix.dir8_tile : ix.dir32_tile) == (int32_t)tile_cap;
-    // dense lists counted from their bitmaps (tiles start at a word boundary)
-    const bool use_bm = ix.bm_slot != nullptr && W.unit_key != nullptr && tile_cap % 128u == 0 &&
+    // dense lists counted from their bitmaps (tiles start at a vector's or a word's boundary)
+    const bool use_bm = ix.bm_slot != nullptr && W.unit_key != nullptr && dense_tile_takes_bitmaps(tile_cap, SMALL) &&
                         (T.dense_bitmaps & (SMALL ? 1 : 2)) != 0;
     for (;;) {
         if (tid == 0) {
