@@ -22,7 +22,7 @@ struct genie_batch {
     cudaStream_t stream = nullptr;
     cudaGraphExec_t gexec = nullptr;
     bool graph_valid = false;
-    bool graph_planes = false;       // the graph was captured with the index's planes
+    int64_t graph_planes = 0;        // which planes of the index the graph was captured with (0: none)
     uint32_t need = 0, graph_need = 0;   // LaunchNeed of the batches staged so far, and of the graph
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     cudaEvent_t stage_ev[kStages + 1] = {};
@@ -83,11 +83,16 @@ bool caller_captures(const genie_batch *b, cudaStream_t s) {
 
 int enqueue(genie_batch *b, cudaStream_t s) {
     DeviceContext &ctx = device_context(b->ix->device);
-    const bool planes = b->ix->pl_tiles > 0 && b->tuning.dense_bitmaps && b->ws.planes.p;
+    const PlanesUse use(b->ix);
+    const int64_t planes = b->ix->pl_tiles > 0 && b->tuning.dense_bitmaps && b->ws.planes.p ? b->ix->pl_built.load() : 0;
     // A caller that captures a launch replays it for whatever it stages later:
-    // no kernel is left out.
+    // no kernel is left out, and the planes stay.
     const bool captured = caller_captures(b, s);
     const uint32_t need = captured ? (uint32_t)kNeedAll : b->need;
+    if (captured && planes) {
+        std::lock_guard<std::mutex> g(b->ix->pl_mu);
+        b->ix->pl_held = true;
+    }
     if (b->graph_valid && b->cfg.use_graph && b->graph_planes == planes && (!planes || b->graph_need == need)) {
         cudaError_t e = cudaGraphLaunch(b->gexec, s);
         return e ? cuda_fail(e, "graph launch") : GENIE_OK;
@@ -102,7 +107,7 @@ int enqueue(genie_batch *b, cudaStream_t s) {
         cudaError_t e = cudaGetLastError();
         return e ? cuda_fail(e, "batch launch") : GENIE_OK;
     }
-    if (!b->graph_valid || b->graph_planes != (d.planes != nullptr) || (d.planes && b->graph_need != need)) {
+    if (!b->graph_valid || b->graph_planes != planes || (planes && b->graph_need != need)) {
         b->graph_valid = false;
         if (b->gexec) cudaGraphExecDestroy(b->gexec);
         b->gexec = nullptr;
@@ -121,7 +126,7 @@ int enqueue(genie_batch *b, cudaStream_t s) {
         cudaGraphDestroy(g);
         if (e) return cuda_fail(e, "graph instantiate");
         b->graph_valid = true;
-        b->graph_planes = d.planes != nullptr;
+        b->graph_planes = planes;
         b->graph_need = need;
     }
     cudaError_t e = cudaGraphLaunch(b->gexec, s);

@@ -336,8 +336,8 @@ int build_device_index(const int32_t *values, int64_t n, int32_t d, genie_index 
         return e == cudaErrorMemoryAllocation ? fail(GENIE_ERR_GPU_ALLOC, "device index build: out of memory")
                                               : cuda_fail(e, what);
     };
-    if ((e = cudaMalloc(&d_vals, cells * 4)) || (e = cudaMalloc(&d_bounds, (size_t)d * 8)) ||
-        (e = cudaMalloc(&d_plan, (size_t)d * sizeof(DimPlan))))
+    if ((e = device_alloc((void **)&d_vals, cells * 4)) || (e = device_alloc((void **)&d_bounds, (size_t)d * 8)) ||
+        (e = device_alloc((void **)&d_plan, (size_t)d * sizeof(DimPlan))))
         return give_up("device index build");
     std::vector<int32_t> bounds((size_t)d * 2, INT32_MAX);
     std::fill(bounds.begin() + d, bounds.end(), INT32_MIN);
@@ -384,7 +384,7 @@ int build_device_index(const int32_t *values, int64_t n, int32_t d, genie_index 
         return GENIE_OK;         // beyond a grid: the host builds this index
     }
     const int64_t nk = h.n_keys();
-    if ((e = cudaMalloc(&d_col, cells * 2)) || (e = cudaMalloc(&d_H, (size_t)hist * 4)) ||
+    if ((e = device_alloc((void **)&d_col, cells * 2)) || (e = device_alloc((void **)&d_H, (size_t)hist * 4)) ||
         (e = ix->d_key_off.reserve((size_t)(nk + 1) * 8)) ||
         (e = cudaMemcpy(d_plan, plan.data(), (size_t)d * sizeof(DimPlan), cudaMemcpyHostToDevice)))
         return give_up("device index build");

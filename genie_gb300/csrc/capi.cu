@@ -32,13 +32,22 @@ int cuda_fail(cudaError_t e, const char *what) {
                 cudaGetErrorString(e));
 }
 
+cudaError_t device_alloc(void **p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation && give_back_planes()) {
+        cudaGetLastError();
+        e = cudaMalloc(p, bytes);
+    }
+    return e;
+}
+
 cudaError_t DevBuf::reserve(size_t want) {
     if (want <= bytes) return cudaSuccess;
     if (p) cudaFree(p);
     p = nullptr;
     bytes = 0;
     size_t b = want + want / 4 + 256;
-    cudaError_t e = cudaMalloc(&p, b);
+    cudaError_t e = device_alloc(&p, b);
     if (e == cudaSuccess) bytes = b;
     return e;
 }
@@ -337,6 +346,7 @@ int run_search(genie_index *ix, const genie_queries *q, const std::vector<int64_
     const size_t o_ids = place((size_t)sumk * 4), o_counts = place((size_t)sumk * 4);
     const size_t o_scores = place(out_scores ? (size_t)sumk * 4 : 0);
     const bool small = at <= kCallBytes && ix->host_err != nullptr;
+    const PlanesUse use(ix);
     DevIndex d = index_view(ix, ix->tuning);
     if (d.planes && ws.reserve_planes(Q)) {     // no room: on the lists
         cudaGetLastError();
@@ -430,6 +440,7 @@ using namespace gg;
 
 genie_index::~genie_index() {
     cudaSetDevice(device);
+    forget_planes(this);
     if (stream) cudaStreamDestroy(stream);
     d_ids.release(); d_key_off.release(); d_key_base.release(); d_dim_min.release(); d_dim_max.release();
     d_words.release(); d_key_seg.release(); d_seg_word_off.release(); d_seg_first.release(); d_seg_len.release();
@@ -558,6 +569,7 @@ int genie_index_get_info(const genie_index *ix, genie_index_info *out) {
     out->device_bytes = (int64_t)(ix->d_ids.bytes + ix->d_key_off.bytes + ix->d_key_base.bytes + ix->d_dim_min.bytes +
                                   ix->d_dim_max.bytes + ix->d_words.bytes + ix->d_key_seg.bytes +
                                   ix->d_seg_word_off.bytes + ix->d_seg_first.bytes + ix->d_seg_len.bytes);
+    if (ix->pl_tiles > 0) out->device_bytes += (int64_t)(ix->d_planes.bytes + ix->d_pl_vals.bytes);
     return GENIE_OK;
 }
 

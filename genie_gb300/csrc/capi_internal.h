@@ -18,6 +18,10 @@ namespace gg {
 int fail(int code, const char *fmt, ...);
 int cuda_fail(cudaError_t e, const char *what);
 
+// cudaMalloc; when the device is full, once more after the planes (planes.cu)
+// of the indexes that no call is using have been given back.
+cudaError_t device_alloc(void **p, size_t bytes);
+
 // One growable device allocation.
 struct DevBuf {
     void *p = nullptr;
@@ -73,6 +77,19 @@ DevIndex index_view(genie_index *ix, const Tuning &t);
 void note_search(genie_index *ix, const genie_queries *q, const Tuning &t);
 // Whether the index's values allow planes, built or not.
 bool may_have_planes(genie_index *ix);
+// Frees the planes of the current device's indexes that are not in use; whether
+// there were any.  Their searches go back to the lists, and earn planes anew.
+bool give_back_planes();
+// An index is destroyed.
+void forget_planes(genie_index *ix);
+// Held from an index's view to the launch of what uses it.
+struct PlanesUse {
+    genie_index *ix;
+    explicit PlanesUse(genie_index *index);
+    ~PlanesUse();
+    PlanesUse(const PlanesUse &) = delete;
+    PlanesUse &operator=(const PlanesUse &) = delete;
+};
 // Kernels that a batch may need on an index with planes (LaunchNeed); a batch
 // without them needs kNeedLists.
 uint32_t launch_need(const genie_index *ix, const genie_queries *q);
@@ -128,10 +145,14 @@ struct genie_index {
     gg::DevBuf d_bm_slot, d_bm_rows;
     std::vector<std::pair<int32_t, gg::DevBuf *>> dirs;
     std::atomic<int64_t> pl_bytes{-1};   // what the planes take (0: the index has none, -1: not looked at)
-    int64_t pl_touched = 0;          // posting ids its searches have touched before they were built
+    std::atomic<int64_t> pl_touched{0};  // posting ids its searches have touched before they were built
     std::atomic<int64_t> pl_tiles{0};    // set once built
+    std::atomic<int64_t> pl_built{0};    // how often they have been: a graph holds the pointers of one time
     int64_t pl_row_vec = 0;
     gg::DevBuf d_planes, d_pl_vals;
+    std::mutex pl_mu;                // of the two below; held while the planes are freed
+    int pl_users = 0;                // calls between the index's view and their launches
+    bool pl_held = false;            // a caller captured launches that use the planes
     cudaStream_t stream = nullptr;
     std::mutex mu;                   // serialises searches on this handle's workspace
     gg::Workspace ws;

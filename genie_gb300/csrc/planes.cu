@@ -8,8 +8,8 @@
 // the planes take (values per dim) / 32 times the ids' bytes: eight times for
 // 256 values.  They are built when a quarter of the device memory that is free
 // then holds all that is kept, once per index (note_search), and kept while it
-// lives.  The
-// values themselves are kept too, one byte each, object by object (a 32nd of
+// lives or until an allocation of this library finds the device full
+// (give_back_planes).  The values themselves are kept too, one byte each, object by object (a 32nd of
 // 256 planes): a weighted tile sums its few candidates from them, whose bytes
 // of one object lie in one or two lines, where the planes would cost a line
 // per item and candidate.
@@ -176,6 +176,10 @@ int64_t planes_bytes(const genie_index *ix) {
     return tiles * rows * row_vec * 16;
 }
 
+// The indexes that have their planes.
+std::mutex g_with_planes_mu;
+std::vector<genie_index *> g_with_planes;
+
 bool build(genie_index *ix) {
     const HostIndex &h = ix->host;
     const int64_t n = h.n_objects, nk = h.n_keys();
@@ -237,11 +241,52 @@ bool build(genie_index *ix) {
         return false;
     }
     ix->pl_row_vec = row_vec;
+    std::lock_guard<std::mutex> g(g_with_planes_mu);
+    g_with_planes.push_back(ix);
+    ++ix->pl_built;
     ix->pl_tiles = tiles;
     return true;
 }
 
 }  // namespace
+
+// A launch in flight has its pointers already, so the device is waited for; a
+// call that has a view but has not launched counts in pl_users; a batch's own
+// graph is captured again without the planes (enqueue), one of a caller's
+// cannot be, so those keep them.
+bool give_back_planes() {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    std::lock_guard<std::mutex> g(g_with_planes_mu);
+    bool any = false;
+    for (size_t i = g_with_planes.size(); i-- > 0;) {
+        genie_index *ix = g_with_planes[i];
+        std::lock_guard<std::mutex> use(ix->pl_mu);
+        if (ix->device != dev || ix->pl_users > 0 || ix->pl_held || cudaDeviceSynchronize()) continue;
+        ix->d_planes.release();
+        ix->d_pl_vals.release();
+        ix->pl_touched = 0;
+        ix->pl_tiles = 0;
+        g_with_planes.erase(g_with_planes.begin() + (std::ptrdiff_t)i);
+        any = true;
+    }
+    return any;
+}
+
+void forget_planes(genie_index *ix) {
+    std::lock_guard<std::mutex> g(g_with_planes_mu);
+    g_with_planes.erase(std::remove(g_with_planes.begin(), g_with_planes.end(), ix), g_with_planes.end());
+}
+
+PlanesUse::PlanesUse(genie_index *index) : ix(index) {
+    std::lock_guard<std::mutex> g(ix->pl_mu);
+    ++ix->pl_users;
+}
+
+PlanesUse::~PlanesUse() {
+    std::lock_guard<std::mutex> g(ix->pl_mu);
+    --ix->pl_users;
+}
 
 // Building the planes takes about as long as counting four times their bytes
 // of posting ids without them (260,000 x 128, 1.1 GB of planes: build 1 ms,

@@ -79,7 +79,7 @@ typedef struct {
     int64_t n_segments;    /* compressed segments (0 when uncompressed) */
     int32_t max_multiplicity; /* most times one id repeats in one list */
     int32_t max_segment;   /* segment length bound of a compressed index */
-    int64_t device_bytes;  /* HBM held by the index */
+    int64_t device_bytes;  /* HBM held by the index, its planes included while it has them */
 } genie_index_info;
 
 /* Build a resident index from a row-major n_objects x n_dims value matrix.

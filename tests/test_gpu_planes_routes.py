@@ -62,3 +62,41 @@ def test_autotuning_keeps_the_planes(genie, weighted):
     genie.search(table, _wide(genie, table))
     b.run(sample)
     assert b.last_stats()[0] == PLANES
+
+
+def test_planes_are_given_back_to_a_failing_allocation(genie, oracle):
+    """An allocation that finds the device full takes the planes back, the
+    searches go on from the lists and earn them again; the planes that a launch
+    captured by its caller reads stay."""
+    import torch
+    table, values = _table(genie)
+    wide, few = _wide(genie, table), _exact(genie, values, 3, 12)
+    expect = oracle.Index(values).search(few.as_oracle_batch())
+    before = genie.Table.info(table).device_bytes
+    b = genie.Batch(table, 3, 36, 10, use_graph=False)
+
+    def run():
+        ids, counts = b.run(few)
+        assert np.array_equal(counts, expect[1]) and np.array_equal(ids, expect[0])
+        return b.last_stats()[0]
+
+    def too_much():      # part results of half a terabyte
+        with pytest.raises(genie.gpu_bad_alloc):
+            genie.Batch(table, 1 << 19, 16, 2048)
+
+    def held():
+        table._info = None
+        return table.info().device_bytes - before
+
+    assert run() == LISTS and held() == 0
+    genie.search(table, wide)
+    assert run() == PLANES and held() > 0
+    too_much()
+    assert held() == 0 and run() == LISTS
+    genie.search(table, wide)
+    assert run() == PLANES and held() > 0
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream, capture_error_mode="thread_local"):
+        b.launch(torch.cuda.current_stream().cuda_stream)
+    too_much()
+    assert held() > 0 and run() == PLANES
