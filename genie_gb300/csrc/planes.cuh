@@ -815,8 +815,13 @@ __device__ uint32_t pl_redo(const DevIndex &ix, const Work &W, const PlQuery &pq
 // Merges every query's keys and writes its results, one CTA per query in turn.
 // Once every tile has been counted, the histogram's bound is the k-th primary
 // itself (its bucket, weighted), so the keys at or above it are k and a few
-// ties: they are collected and sorted.  More than the buffer holds go through
-// the general selection.
+// ties: they are collected and sorted.  When the buffer fills (a few queries
+// with a large k, whose tiles were all counted before any bound was known, and
+// many equal counts) it is sorted and its k-th key becomes the bound: tiles
+// write lower ids first, so little more passes.  Selecting from all of a
+// query's keys again and again with 128 threads took most of the call (k = 500,
+// one query of 16 items in 2,000,000 x 128: 978 us a call, 243 so).  Only a k
+// that leaves the buffer no room for a step goes through the general selection.
 __global__ void __launch_bounds__(kPlThreads) k_planes_finish(DevIndex ix, DevQueries Q, Work W) {
     __shared__ PlShared s;
     __shared__ uint64_t cand[kCandCap];
@@ -852,9 +857,11 @@ __global__ void __launch_bounds__(kPlThreads) k_planes_finish(DevIndex ix, DevQu
             }
         }
         __syncthreads();
-        const uint64_t lbk = s.lbk;
-        constexpr uint32_t kAhead = 8;
-        for (uint32_t b = 0; b < n; b += kAhead * kPlThreads) {
+        uint64_t lbk = s.lbk;
+        constexpr uint32_t kAhead = 8, kStep = kAhead * kPlThreads;
+        // what is kept and a step's keys fit the buffer
+        const bool prune = pq.k + kStep <= (uint32_t)kCandCap;
+        for (uint32_t b = 0; b < n; b += kStep) {
             uint64_t key[kAhead];
 #pragma unroll
             for (uint32_t j = 0; j < kAhead; ++j) {
@@ -867,6 +874,18 @@ __global__ void __launch_bounds__(kPlThreads) k_planes_finish(DevIndex ix, DevQu
                     const uint32_t at = atomicAdd(&s.n, 1u);
                     if (at < (uint32_t)kCandCap) cand[at] = key[j];
                 }
+            if (!prune || b + kStep >= n) continue;
+            __syncthreads();
+            const uint32_t have = s.n;
+            if (have + kStep > (uint32_t)kCandCap) {      // more than k
+                const uint32_t np2 = next_pow2(have);
+                for (uint32_t i = have + tid; i < np2; i += kPlThreads) cand[i] = 0ull;
+                bitonic_sort_desc(cand, np2);
+                lbk = cand[pq.k - 1];
+                __syncthreads();
+                if (tid == 0) s.n = pq.k;
+            }
+            __syncthreads();
         }
         __syncthreads();
         uint32_t got = s.n;

@@ -1,0 +1,37 @@
+"""Tables of several tiles: the merge of many tiles' keys.  Every result is a
+whole number and compared exactly."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _ready(genie, values):
+    """A table with its planes built."""
+    t = genie.Table.from_values(values)
+    n, d = values.shape
+    lo, up = int(values.min()), int(values.max())
+    q = 2 + -(-n // 16384) * 2048 * (len(t.layout()["key_offsets"]) + 1) // (n * d)
+    genie.search(t, genie.QueryBatch(np.arange(q + 1) * d, np.tile(np.arange(d), q), np.full(q * d, lo), np.full(q * d, up), 1))
+    return t
+
+
+def _batch(genie, rng, q, m, d, low, up, k, weighted):
+    w = rng.uniform(0.5, 2.0, q * m).astype(np.float32) if weighted else None
+    dim = np.concatenate([rng.permutation(d)[:m] for _ in range(q)])
+    return genie.QueryBatch(np.arange(q + 1) * m, dim, low, up, k, w, np.ones(q, np.uint8) if weighted else None)
+
+
+@pytest.mark.parametrize("k", [500, 1024, 1025, 2048])
+@pytest.mark.parametrize("n", [400_000, 700_001])
+def test_merge_of_many_keys(genie, oracle, n, k):
+    """A query alone: all its tiles write k keys each, most of them tied, far
+    more than the merge's buffer holds at once (beyond k = 1,024 it selects)."""
+    rng = np.random.default_rng(n + k)
+    values = rng.integers(0, 9, size=(n, 8)).astype(np.int32)
+    table = _ready(genie, values)
+    low = rng.integers(0, 7, 8)
+    qb = _batch(genie, rng, 1, 8, 8, low, low + 2, k, False)
+    expect = oracle.Index(values).search(qb.as_oracle_batch())
+    got = genie.search(table, qb)
+    assert np.array_equal(got[1], expect[1]) and np.array_equal(got[0], expect[0])
