@@ -267,7 +267,7 @@ int genie_batch_create(genie_index *ix, const genie_batch_config *cfg, genie_bat
     // what the planes need is there before they are: a launch allocates nothing
     // and every launch of a batch, also one its caller captured, uses the same
     // buffers.  Without the memory for it the batch stays on the lists.
-    if (may_have_planes(ix) && b->ws.reserve_planes(Q)) {
+    if (may_have_planes(ix) && b->ws.reserve_planes(Q, K, ix->host.n_objects)) {
         cudaGetLastError();
         b->ws.planes.release();
     }

@@ -117,9 +117,16 @@ cudaError_t Workspace::reserve(int64_t Q, int64_t items, int64_t units, int64_t 
     return cudaSuccess;
 }
 
-cudaError_t Workspace::reserve_planes(int64_t Q) {
-    // a few queries of many tiles write more than 64 parts' keys each
-    cudaError_t e = scratch.reserve(8 << 20);
+// A query's tiles write up to k keys each, and do where its objects tie (few
+// items) so that no bound tells them apart; a region that is too small costs a
+// recount of the table by one block (512 weighted queries of four items, k =
+// 500, 2,000,000 objects: 12.4 ms a batch with 64 k keys a query, 2.0 with all
+// 123 k).  So there is room for all of them, unless that is more than
+// kPlRegions.
+constexpr size_t kPlRegions = size_t(512) << 20;
+cudaError_t Workspace::reserve_planes(int64_t Q, int64_t sumk, int64_t n_objects) {
+    const size_t all = (size_t)sumk * (size_t)((n_objects + kPlTile - 1) / kPlTile) * 8;
+    cudaError_t e = scratch.reserve(std::min(kPlRegions, all));
     if (!e) e = planes.reserve((size_t)Q * (8 + 256 * 4 + 4) + 64);
     return e;
 }
@@ -348,7 +355,7 @@ int run_search(genie_index *ix, const genie_queries *q, const std::vector<int64_
     const bool small = at <= kCallBytes && ix->host_err != nullptr;
     const PlanesUse use(ix);
     DevIndex d = index_view(ix, ix->tuning);
-    if (d.planes && ws.reserve_planes(Q)) {     // no room: on the lists
+    if (d.planes && ws.reserve_planes(Q, sumk, ix->host.n_objects)) {     // no room: on the lists
         cudaGetLastError();
         ws.planes.release();
         d.planes = nullptr;

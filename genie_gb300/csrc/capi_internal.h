@@ -55,7 +55,7 @@ struct Workspace {
     cudaError_t reserve(int64_t Q, int64_t items, int64_t units, int64_t sumk, bool io = true);
     // what a search with an index's planes needs beside; before reserve() and
     // view() (when it fails it may have freed the scratch)
-    cudaError_t reserve_planes(int64_t Q);
+    cudaError_t reserve_planes(int64_t Q, int64_t sumk, int64_t n_objects);
     void release();
     Work view(int64_t Q, bool scores) const;
 };

@@ -5,6 +5,8 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
+PLANES = 3        # launches: plan, tiles, merge
+
 
 def _ready(genie, values):
     """A table with its planes built."""
@@ -35,3 +37,21 @@ def test_merge_of_many_keys(genie, oracle, n, k):
     expect = oracle.Index(values).search(qb.as_oracle_batch())
     got = genie.search(table, qb)
     assert np.array_equal(got[1], expect[1]) and np.array_equal(got[0], expect[0])
+
+
+def test_more_keys_than_the_largest_regions(genie, oracle):
+    """Ties in every tile of a batch whose keys do not all fit: the queries are
+    counted again, tile by tile."""
+    rng = np.random.default_rng(5)
+    n, q, k = 2_000_000, 2600, 400
+    values = rng.integers(0, 50, size=(n, 2)).astype(np.int32)
+    table = _ready(genie, values)
+    qb = genie.QueryBatch(np.arange(q + 1), np.zeros(q, np.int32), np.arange(q) % 40, np.arange(q) % 40, k)
+    expect = oracle.Index(values).search(genie.QueryBatch(np.arange(41), np.zeros(40, np.int32), np.arange(40),
+                                                          np.arange(40), k).as_oracle_batch())
+    b = genie.Batch(table, q, q, k)
+    ids, counts = b.run(qb)
+    assert b.last_stats()[0] == PLANES
+    at = np.arange(q) % 40
+    assert np.array_equal(ids.reshape(q, k), expect[0].reshape(40, k)[at])
+    assert np.array_equal(counts.reshape(q, k), expect[1].reshape(40, k)[at])
