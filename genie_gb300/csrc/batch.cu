@@ -72,6 +72,7 @@ DevQueries device_queries(const genie_batch *b) {
     q.uniform_k = 0;
     q.out_off = (const int64_t *)b->ws.out_off.p;
     q.dyn = (const uint32_t *)b->dyn.p;
+    q.route = 0;
     return q;
 }
 
@@ -147,7 +148,6 @@ int stage_async(genie_batch *b, const genie_queries *q, cudaStream_t s) {
         if (k > b->cfg.max_k) return fail(GENIE_ERR_INVALID_ARG, "k=%u exceeds the batch capacity %u", k, b->cfg.max_k);
     }
     note_search(b->ix, q, b->tuning);
-    b->need |= launch_need(b->ix, q);
     // The caller's item arrays are uploaded from where they are: a copy from
     // pageable memory returns once the source may be reused, and on a
     // coherently attached host it moves the bytes without a staging memcpy,
@@ -162,6 +162,9 @@ int stage_async(genie_batch *b, const genie_queries *q, cudaStream_t s) {
     b->h_dyn[0] = (uint32_t)Q;
     b->h_dyn[1] = q->uniform_k;
     b->h_dyn[2] = exact ? 1u : 0u;
+    const PlanesPlan plan = planes_plan(b->ix, q);
+    b->need |= plan.need;
+    b->h_dyn[3] = plan.route;
     cudaError_t e = cudaSuccess;
     Workspace &ws = b->ws;
     auto h2d = [&](void *dst, const void *src, size_t n) {
@@ -175,7 +178,7 @@ int stage_async(genie_batch *b, const genie_queries *q, cudaStream_t s) {
     h2d(ws.weighted.p, weighted ? (const void *)q->weighted : (const void *)b->h_weighted, Q);
     h2d(ws.k.p, b->h_k, Q * 4);
     h2d(ws.out_off.p, b->h_out_off, (Q + 1) * 8);
-    h2d(b->dyn.p, b->h_dyn, 12);
+    h2d(b->dyn.p, b->h_dyn, 16);
     if (e) return cuda_fail(e, "batch upload");
     b->staged_q = (int32_t)Q;
     b->staged_sumk = out_off[Q];

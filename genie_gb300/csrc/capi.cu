@@ -368,6 +368,8 @@ int run_search(genie_index *ix, const genie_queries *q, const std::vector<int64_
     dq.n_queries = (int32_t)Q;
     dq.uniform_k = q->uniform_k;
     dq.dyn = nullptr;
+    const PlanesPlan plan = planes_plan(ix, q);
+    dq.route = plan.route;
     unsigned char *dev = (unsigned char *)ws.call.p, *host = (unsigned char *)ix->host_err + 256;
     if (small) {
         memcpy(host + o_item_off, q->item_off, (size_t)(Q + 1) * 8);
@@ -422,7 +424,7 @@ int run_search(genie_index *ix, const genie_queries *q, const std::vector<int64_
         w.out_cap = sumk;
     }
     ix->last_launches = launch_match(d, dq, w, ix->tuning, ctx.num_sms, s, nullptr,
-                                     launch_need(ix, q) | (small ? kCtrZeroed : 0u));
+                                     plan.need | (small ? kCtrZeroed : 0u));
     if ((e = cudaGetLastError())) return cuda_fail(e, "match launch");
     ix->call_results = -1;
     if (small) {

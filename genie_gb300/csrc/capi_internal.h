@@ -90,9 +90,13 @@ struct PlanesUse {
     PlanesUse(const PlanesUse &) = delete;
     PlanesUse &operator=(const PlanesUse &) = delete;
 };
-// Kernels that a batch may need on an index with planes (LaunchNeed); a batch
-// without them needs kNeedLists.
-uint32_t launch_need(const genie_index *ix, const genie_queries *q);
+// How a batch is counted on an index with planes: the kernels to launch
+// (LaunchNeed; a batch without planes needs kNeedLists) and the PlanesRoute that
+// the plan kernel goes by.
+struct PlanesPlan {
+    uint32_t need, route;
+};
+PlanesPlan planes_plan(const genie_index *ix, const genie_queries *q);
 
 // Asynchronous steps of one batch for the serving loop (batch.cu): stage,
 // launch and download on the batch's own stream; poll; copy the results out.

@@ -40,19 +40,59 @@ constexpr uint32_t kPlAnyK = 128;
 constexpr uint32_t kPlGroup8 = 72;
 constexpr uint32_t kPlUnitMax = 31;
 constexpr uint32_t kPlBoundMax = 2047;
-// Whether a query of an index with planes is counted with them: m items that
-// end at item_end, counts of at most eight bits (one value per object and dim:
-// at most m).  Weighted results must fit a tile's buffer, and beyond kPlAnyK
-// few of the objects may be results: a tile sums its candidates, a few times
-// k, one by one (64 queries of 8-120 items, half k = 10 and half k = 500, on
-// 20,000 objects: 209 us with lists and 328 with planes; on 500,000: 680 and
-// 602).  The plan decides by it on the device, and the host by the same rule
-// which kernels to launch.
+// Whether a query of an index with planes may be counted with them: m items
+// that end at item_end, counts of at most eight bits (one value per object and
+// dim: at most m).  Weighted results must fit a tile's buffer, and beyond
+// kPlAnyK few of the objects may be results: a tile sums its candidates, a few
+// times k, one by one (64 queries of 8-120 items, half k = 10 and half k = 500,
+// on 20,000 objects: 209 us with lists and 328 with planes).
 __host__ __device__ inline bool planes_take(int64_t m, int64_t item_end, bool weighted, uint32_t k, int32_t n_dims,
                                             int64_t n_objects) {
     if (m > (int64_t)kPlMaxItems || item_end > 0xFFFFFFFFll) return false;
     return !weighted || (n_dims <= 65536 && (k <= kPlAnyK || (k <= kPlMaxWeightedK && (int64_t)k * 256 <= n_objects)));
 }
+// Which of them are: those that the planes count sooner than the lists do.  An
+// item costs two plane rows a tile whatever it covers, and a tile a selection;
+// the lists cost its posting ids, so the planes lose where these are few (512
+// weighted queries of three rare values on 2,000,000 objects: 861 us on planes,
+// 162 on lists), or many results are wanted of few queries, whose tiles all run
+// before any bound is known.  Device time of a query in picoseconds, fitted to
+// 6,016 batches timed both ways (20,000 to 2,000,000 objects, 1 to 512 queries
+// of 1 to 120 items, k 10 to 500, items of 1/20,000 to 1/7 of the objects): the
+// side it picks takes 1.4 % longer than the faster one on the mean unweighted,
+// 1.7 % weighted, and over 10 % longer than the lists for 62 of them.
+struct PlanesCost {
+    int64_t planes, dense0, objects;
+    bool weighted;
+    __host__ __device__ PlanesCost(int64_t m, bool w, uint32_t k, int64_t n, int64_t nq) : objects(n), weighted(w) {
+        const int64_t tiles = (n + kPlTile - 1) / kPlTile;
+        // tiles of the query that run at once: its share of 152 x 4 blocks
+        const int64_t share = nq > 0 ? (608 + nq - 1) / nq : 608, at_once = tiles < share ? tiles : share;
+        // a batch whose tiles run in one or two rounds leaves the lists' kernels
+        // more of the chip idle than the planes'
+        const int64_t alone = nq * tiles > 1216 ? 1 : w ? 4 : 2;
+        planes = w ? tiles * (8100 + 230 * m) / alone + 1500 * (int64_t)k + at_once * k * k * 17 / 20
+                   : tiles * (2800 + 160 * m) / alone + at_once * k * 36;
+        // the counter tiles; few unweighted items tie a lot
+        dense0 = w ? 595000 + tiles * (26000 + 140 * m) : 225000 + tiles * (10300 + 46 * m + (m <= 2 ? 40000 : 0));
+    }
+    // a query that touches `total` posting ids, on the lists
+    __host__ __device__ int64_t lists(int64_t total) const {
+        const int64_t dense = dense0 + (weighted ? total / 2 : total / 6);
+        // a hash table of 16 parts at half load takes at most
+        if (total > (weighted ? 90112 : 180224) || total * 4 > objects * 3) return dense;
+        if (weighted || objects > 1179648 || total > (int64_t)kBmMaxIds) return total * (weighted ? 40 : 24);
+        // the bitmap kernel, unless more ids repeat than its table holds
+        return total * total > 2048 * objects ? dense : total * 5;
+    }
+};
+// A batch is counted one way as a whole, by a sample of its queries
+// (planes_plan), or, where that saves more than kPlBothPs of a second set of
+// kernels running after the first (64 weighted queries of four items, k = 500,
+// split between both on 200,000 objects: 766 us, 384 with lists alone and 394
+// with planes), each query its own way, as the plan kernel finds.
+enum PlanesRoute : uint32_t { kRoutePlanes = 0, kRouteLists = 1, kRouteEach = 2 };
+constexpr int64_t kPlBothPs = 60000000;
 // rows of a tile behind its keys' rows: no object, and every object
 constexpr uint32_t kPlExtraRows = 2;
 // zero bytes behind the posting ids of a plain index: 32 ids read from the
@@ -124,8 +164,10 @@ struct DevQueries {
     const int64_t *out_off;
     // optional device-side size of a captured batch: dyn[0] = queries in this
     // run (<= n_queries, the capacity), dyn[1] = uniform k, dyn[2] = 1 when
-    // every item is exact (up = low; the up array is not sent)
+    // every item is exact (up = low; the up array is not sent), dyn[3] =
+    // PlanesRoute
     const uint32_t *dyn;
+    uint32_t route;            // PlanesRoute of the batch when dyn is null
 };
 
 // Per-query plan written by k_plan.

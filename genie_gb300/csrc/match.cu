@@ -105,13 +105,10 @@ __global__ void __launch_bounds__(kPlanThreads, 8) k_plan(DevIndex ix, DevQuerie
     if (s_oob) return;
     const bool weighted = Q.weighted && Q.weight && Q.weighted[q];
     const bool exact = Q.dyn && Q.dyn[2];      // a batch of exact items sends no upper bounds
-    // Counted from the cumulative planes whenever the index has them: a range
-    // item costs two rows of 1/8 byte an object whatever it covers, against 4
-    // bytes and a shared atomic per posting id elsewhere.  Even exact items
-    // (1 % of the objects each) are faster there than hashed: 260,000 x 128,
-    // 256 queries of 8-128 items, a quarter of them exact, 494 us before (125
-    // of them hashing the exact ones) and 140 us.
-    const bool planes = ix.planes != nullptr && W.lbk != nullptr && planes_take(m, i1, weighted, k, ix.n_dims, ix.n_objects);
+    // May be counted from the cumulative planes; whether it is may depend on its total.
+    const uint32_t route = Q.dyn ? Q.dyn[3] : Q.route;
+    const bool may = ix.planes != nullptr && W.lbk != nullptr && route != kRouteLists &&
+                     planes_take(m, i1, weighted, k, ix.n_dims, ix.n_objects);
     if (tid == 0) {
         s_total = 0;
         s_units = 0;
@@ -147,7 +144,7 @@ __global__ void __launch_bounds__(kPlanThreads, 8) k_plan(DevIndex ix, DevQuerie
     int64_t k0_first = 0, a_first = 0, e_first = 0;     // a, e: list offsets around the keys
     uint32_t nk_first = 0, inc_first = 1;
     // planes of low - 1 and up of this thread's item (byte offsets in a tile)
-    const uint32_t pl_row = planes ? (uint32_t)ix.pl_row_vec * 16u : 0u;
+    const uint32_t pl_row = may ? (uint32_t)ix.pl_row_vec * 16u : 0u;
     uint32_t test = 0;       // its dim, low and width, low relative to the dim's least value
     uint2 rows = make_uint2((uint32_t)ix.pl_keys * pl_row, ((uint32_t)ix.pl_keys + 1u) * pl_row);
     for (int64_t i = i0 + tid; i < i1; i += nt) {
@@ -164,7 +161,7 @@ __global__ void __launch_bounds__(kPlanThreads, 8) k_plan(DevIndex ix, DevQuerie
                 a = ix.key_off[k0];
                 e = ix.key_off[k0 + nk];
                 total += (uint64_t)(e - a);
-                if (planes) {
+                if (may) {
                     if (lo > mn) rows.x = (uint32_t)(k0 - 1) * pl_row;
                     if (hi < mx) rows.y = (uint32_t)(k0 + nk - 1) * pl_row;
                     test = (uint32_t)d << 16 | (uint32_t)(lo - mn) << 8 | (uint32_t)(hi - lo);
@@ -177,7 +174,7 @@ __global__ void __launch_bounds__(kPlanThreads, 8) k_plan(DevIndex ix, DevQuerie
         // of the query is, the query's units are its items and nothing more
         // is written.  Otherwise the query takes a unit range past the
         // batch's items and these slots, in its own item range, stay unread.
-        if (nk <= 1 && i < W.units_cap && !planes) {
+        if (nk <= 1 && i < W.units_cap && !may) {
             if (ix.codec) {
                 a = nk ? ix.key_seg[k0] : 0;
                 e = nk ? ix.key_seg[k0 + 1] : 0;
@@ -216,6 +213,17 @@ __global__ void __launch_bounds__(kPlanThreads, 8) k_plan(DevIndex ix, DevQuerie
     __syncthreads();
     const int64_t unit0 = (int64_t)s_unit0, n_units = single ? (int64_t)m : (int64_t)s_units;
     total = s_total;
+    bool planes = may;
+    if (may && route == kRouteEach) {
+        const PlanesCost cost(m, weighted, k, ix.n_objects, nq);
+        planes = cost.planes <= cost.lists((int64_t)total);
+    }
+    if (may && !planes && i0 + tid < i1 && nk_first <= 1 && i0 + tid < W.units_cap) {      // its one item, as above
+        W.span_start[i0 + tid] = a_first;
+        W.span_len[i0 + tid] = e_first - a_first;
+        W.inc[i0 + tid] = inc_first;
+        if (W.unit_key) W.unit_key[i0 + tid] = (uint32_t)k0_first;
+    }
     const bool fits = unit0 + n_units <= W.units_cap;
     if (tid == 0 && !fits) atomicOr(&W.ctr[kCtrError], kErrUnits);
     // one unit per covered list (a query with several lists in one item)

@@ -157,6 +157,7 @@ extern "C" int genie_search_noalloc(genie_index *ix, const genie_queries *q, con
     dq.uniform_k = q->uniform_k;
     dq.out_off = out_off;
     dq.dyn = nullptr;
+    dq.route = kRouteLists;
     cudaStream_t s = (cudaStream_t)stream;
     // the work counters must start at zero (launch_match clears them); the
     // per-query completion counters are reset by the plan kernel

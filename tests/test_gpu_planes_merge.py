@@ -55,3 +55,26 @@ def test_more_keys_than_the_largest_regions(genie, oracle):
     at = np.arange(q) % 40
     assert np.array_equal(ids.reshape(q, k), expect[0].reshape(40, k)[at])
     assert np.array_equal(counts.reshape(q, k), expect[1].reshape(40, k)[at])
+
+
+@pytest.mark.parametrize("weighted", [False, True])
+def test_ties_below_k_in_every_tile(genie, oracle, weighted):
+    """420 objects of one value a tile, 512 wanted: no tile alone bounds the
+    query, and all 123 write more keys than its region holds."""
+    rng = np.random.default_rng(6)
+    n, q, k, v = 2_000_000, 2100, 512, 39
+    values = rng.integers(0, v, size=(n, 2)).astype(np.int32)
+    table = _ready(genie, values)
+    at = np.arange(q) % v
+    w = np.full(q, 1.5, np.float32) if weighted else None
+    wf = np.ones(q, np.uint8) if weighted else None
+    few = slice(0, v)
+    qb = genie.QueryBatch(np.arange(q + 1), np.zeros(q, np.int32), at, at, k, w, wf)
+    one = genie.QueryBatch(np.arange(v + 1), np.zeros(v, np.int32), at[few], at[few], k, None if w is None else w[few],
+                           None if wf is None else wf[few])
+    expect = oracle.Index(values).search(one.as_oracle_batch())
+    b = genie.Batch(table, q, q, k)
+    got = b.run(qb, scores=True)
+    assert b.last_stats()[0] == PLANES
+    for x, y in zip(got, expect):
+        assert np.array_equal(x.reshape(q, k), y.reshape(v, k)[at])
