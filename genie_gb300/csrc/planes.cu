@@ -290,8 +290,8 @@ PlanesUse::~PlanesUse() {
 
 namespace {
 
-// What a batch touches is told from at most 32 of its queries and 16 items of
-// each (2 us): every item looked at took 3 us of a 130 us batch of 12 queries.
+// What a batch touches is told from at most 16 of its queries and 8 items of
+// each (1 us): every item looked at took 3 us of a 130 us batch of 12 queries.
 // One of every group, wherever in it, so that no pattern of the caller's falls
 // in step with them.
 struct Sample {
@@ -303,7 +303,7 @@ struct Sample {
 
 int64_t sampled_ids(const HostIndex &h, const genie_queries *q, int64_t i) {
     const int64_t a = q->item_off[i];
-    const Sample s(q->item_off[i + 1] - a, 16);
+    const Sample s(q->item_off[i + 1] - a, 8);
     int64_t total = 0;
     for (int64_t g = 0; g * s.step < s.n; ++g) {
         const int64_t j = a + s.at(g);
@@ -329,7 +329,7 @@ void note_search(genie_index *ix, const genie_queries *q, const Tuning &t) {
     if (ix->pl_bytes == 0 || ix->pl_tiles > 0) return;
     const HostIndex &h = ix->host;
     const int64_t enough = ix->pl_bytes;       // ids, of four bytes
-    const Sample s(q->n_queries, 32);
+    const Sample s(q->n_queries, 16);
     for (int64_t g = 0; g * s.step < s.n && ix->pl_touched < enough; ++g)
         ix->pl_touched += sampled_ids(h, q, s.at(g)) * s.of(g);
     if (ix->pl_touched >= enough && !build(ix)) ix->pl_bytes = 0;
@@ -361,7 +361,7 @@ PlanesPlan planes_plan(const genie_index *ix, const genie_queries *q) {
     plan.route = kRoutePlanes;
     if (h.n_objects > (int64_t)kPlTile) {        // a table of one tile has planes no slower than its lists throughout
         int64_t planes = others ? kPlBothPs : 0, lists = 0, each = kPlBothPs;
-        const Sample s(q->n_queries, 32);
+        const Sample s(q->n_queries, 16);
         for (int64_t g = 0; g * s.step < s.n; ++g) {
             if (!takes(s.at(g), w, k, m)) continue;
             const PlanesCost cost(m, w, k, h.n_objects, q->n_queries);

@@ -861,19 +861,23 @@ __global__ void __launch_bounds__(kPlThreads) k_planes_finish(DevIndex ix, DevQu
         constexpr uint32_t kAhead = 8, kStep = kAhead * kPlThreads;
         // what is kept and a step's keys fit the buffer
         const bool prune = pq.k + kStep <= (uint32_t)kCandCap;
-        for (uint32_t b = 0; b < n; b += kStep) {
-            uint64_t key[kAhead];
+        uint64_t key[kAhead];
+        const auto load = [&](uint32_t b) {
 #pragma unroll
             for (uint32_t j = 0; j < kAhead; ++j) {
                 const uint32_t i = b + j * kPlThreads + tid;
                 key[j] = i < n ? __ldcg(pq.region + i) : 0ull;
             }
+        };
+        load(0);
+        for (uint32_t b = 0; b < n; b += kStep) {
 #pragma unroll
             for (uint32_t j = 0; j < kAhead; ++j)
                 if (key[j] && key[j] >= lbk) {
                     const uint32_t at = atomicAdd(&s.n, 1u);
                     if (at < (uint32_t)kCandCap) cand[at] = key[j];
                 }
+            load(b + kStep);
             if (!prune || b + kStep >= n) continue;
             __syncthreads();
             const uint32_t have = s.n;
