@@ -5,7 +5,8 @@
 // H2D of the compiled spans, match_AT, a host-synchronising overflow check,
 // heap_count_topk with cudaMalloc/cudaFree, D2H (matching/knn.cu:106-183,
 // match.cu:224-464).  Here the batch size lives in device memory, so the same
-// graph (memset + plan + four persistent kernels) serves every batch.
+// graph (memset, plan and the persistent kernels of the lists, of an index's
+// planes, or both) serves every batch that needs no other kernels.
 #include "capi_internal.h"
 
 #include <cstring>

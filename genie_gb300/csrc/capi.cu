@@ -336,8 +336,7 @@ int run_search(genie_index *ix, const genie_queries *q, const std::vector<int64_
     // A small call is packed: inputs and zeroed counters in one upload, error
     // word and results in one download, both through pinned memory (a lookup in
     // 1,000 x 128: 60 us with eight uploads from and three downloads to
-    // pageable memory and a memset, 42 us so).  A larger one is not: copying
-    // it once more on the host costs more than its copies do.
+    // pageable memory and a memset, 42 us so).
     size_t at = 0;
     auto place = [&](size_t n) {
         const size_t o = at;

@@ -36,7 +36,11 @@ constexpr uint32_t kPlMaxItems = 255;
 constexpr uint32_t kPlMaxWeightedK = 512;
 constexpr uint32_t kPlAnyK = 128;
 // weighted queries there: items up to which a weight group is 8 (else 16), the
-// largest unit weight, and the largest bound (eleven planes)
+// largest unit weight, and the largest bound (eleven planes).  512 queries of
+// 24 / 56 / 72 items on 500,000 objects: 646 / 760 / 852 us a batch, 929 / 868 /
+// 984 with groups of 16; of 80 / 120 items 960 / 1,061, 878 / 1,019 with groups
+// of 8 (1,024 queries of 8 to 128 items on 4,000,000 objects: 7.9 ms either way,
+// 8.8 with groups of 16 throughout).
 constexpr uint32_t kPlGroup8 = 72;
 constexpr uint32_t kPlUnitMax = 31;
 constexpr uint32_t kPlBoundMax = 2047;

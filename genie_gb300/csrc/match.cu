@@ -49,7 +49,8 @@ constexpr int kPlanThreads = 256;
 // CTA, and parts whose share of the index (4 bytes an id, about one
 // compressed) stays within kPartSlice, which L2 keeps while the batch counts
 // them (short texts, 1,000,000 x 32, 1,024 queries: 1.38 ms with a tile a
-// part, 1.03 with the query whole).  Every dense query of one counter width
+// part, 1.03 with the query whole; a call 1.08 ms with kPartSlice, 1.27 with a
+// quarter of it and 1.09 with four times).  Every dense query of one counter width
 // has the same number, so that the dense kernel can take its work part-major
 // (take_dense).
 constexpr int64_t kPartSlice = 48 << 20;

@@ -41,8 +41,9 @@
 // scratch.  lbk[q], a lower bound on the query's final k-th key, prunes: a
 // tile holding k objects raises it to its own k-th key, and a histogram of
 // the primaries written so far bounds it as tiles finish.  k_planes_finish
-// merges.  A region that is too small (many ties, few bounds) makes it redo
-// the query alone, tile by tile, compacting the region.  A table of one tile
+// merges.  A region holds k keys of every tile while the batch's fit 512 MB; one
+// that is too small (many ties, few bounds) makes it redo the query alone, tile
+// by tile, compacting the region.  A table of one tile
 // needs neither: its block writes the results.
 #pragma once
 
