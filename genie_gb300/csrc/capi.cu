@@ -122,11 +122,16 @@ cudaError_t Workspace::reserve(int64_t Q, int64_t items, int64_t units, int64_t 
 // recount of the table by one block (512 weighted queries of four items, k =
 // 500, 2,000,000 objects: 12.4 ms a batch with 64 k keys a query, 2.0 with all
 // 123 k).  So there is room for all of them, unless that is more than
-// kPlRegions.
+// kPlRegions or an eighth of the free device memory.
 constexpr size_t kPlRegions = size_t(512) << 20;
 cudaError_t Workspace::reserve_planes(int64_t Q, int64_t sumk, int64_t n_objects) {
-    const size_t all = (size_t)sumk * (size_t)((n_objects + kPlTile - 1) / kPlTile) * 8;
-    cudaError_t e = scratch.reserve(std::min(kPlRegions, all));
+    size_t regions = std::min(kPlRegions, (size_t)sumk * (size_t)((n_objects + kPlTile - 1) / kPlTile) * 8);
+    if (regions > scratch.bytes) {
+        size_t free_b = 0, total_b = 0;
+        if (cudaMemGetInfo(&free_b, &total_b)) cudaGetLastError();
+        regions = std::min(regions, free_b / 8);
+    }
+    cudaError_t e = scratch.reserve(regions);
     if (!e) e = planes.reserve((size_t)Q * (8 + 256 * 4 + 4) + 64);
     return e;
 }
