@@ -359,7 +359,11 @@ PlanesPlan planes_plan(const genie_index *ix, const genie_queries *q) {
         else others = true;
     if (!kinds) return plan;
     plan.route = kRoutePlanes;
-    if (h.n_objects > (int64_t)kPlTile) {        // a table of one tile has planes no slower than its lists throughout
+    // a table of one tile has planes no slower than its lists throughout, but for
+    // the lists' kernels that other queries of the batch need (49 weighted
+    // queries on 5,072 objects, half k = 10 and half 500: 180 us both ways, 160
+    // on lists)
+    if (h.n_objects > (int64_t)kPlTile || others) {
         int64_t planes = others ? kPlBothPs : 0, lists = 0, each = kPlBothPs;
         const Sample s(q->n_queries, 16);
         for (int64_t g = 0; g * s.step < s.n; ++g) {

@@ -119,6 +119,16 @@ def test_limits_on_one_tile(genie, oracle, items, span, k, weighted, launches):
     assert _run(genie, oracle, table, values, qb) == launches
 
 
+def test_few_queries_beside_ones_of_the_lists(genie, oracle):
+    """Every other of 48 weighted queries wants more results than the planes of
+    a small table give: all go by the lists, whose kernels run anyway."""
+    rng = np.random.default_rng(3)
+    values, table = _one_tile(genie, rng, 5_000, 24, 50)
+    low = rng.integers(0, 40, 48 * 20)
+    k = np.where(np.arange(48) % 2, 500, 10).astype(np.uint32)
+    assert _run(genie, oracle, table, values, _batch(genie, rng, 48, 20, 24, low, low + 6, k, True)) == LISTS
+
+
 @pytest.mark.parametrize("k,launches", [(512, PLANES), (513, LISTS)])
 def test_most_weighted_results(genie, oracle, k, launches):
     """Of many objects 512 weighted results, for queries that touch most of them."""
